@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kGenBlock) k_generate(Wave wv, Views vs, float
 #define CPT_EXTEND_MIN_BLOCKS (1024 / CPT_EXTEND_BLOCK)  // 32 warps per SM: 64 registers
 #endif
 // kWide: every view's wide tree (cpt_lbvh_wide) instead of its binary nodes.
-static_assert(kWideSmemStack * 2 == kSmemStack, "wide and binary stacks share the shared-memory buffer");
+static_assert(kWideSmemStack * 2 <= kSmemStack, "wide and binary stacks share the shared-memory buffer");
 template <bool kStats, bool kOneView, bool kWide>
 __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(Views vs, const float4* __restrict__ queue,
                                                          const uint32_t* __restrict__ count, float4* __restrict__ hits,
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(
                                                          uint32_t* __restrict__ status, const uint32_t* __restrict__ order,
                                                          uint32_t refill)
 {
-    __shared__ __align__(16) uint32_t s_stack[kSmemStack * kExtendBlock];
+    __shared__ __align__(16) uint32_t s_stack[(kWide ? 2 * kWideSmemStack : kSmemStack) * kExtendBlock];
     const uint32_t n = *count;
     bool overflow = false;
     uint32_t nn = 0, nt = 0;
@@ -303,11 +303,9 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(
             tr = vs.v[vi].wide_tris;
             return vs.v[vi].wide_nodes;
         };
-        persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false>(
+        persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false, !kStats>(
             wide_of, queue, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, order,
-            [&](uint32_t ray, const WideState& s) {
-                hits[ray] = make_float4(s.best.t, s.best.u, s.best.v, __uint_as_float(s.best.tri));
-            },
+            WideHits{hits},
             refill);
         if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
         if (kStats && ray_counts) {
@@ -645,6 +643,25 @@ __global__ void __launch_bounds__(kShadeBlock) k_shade(Views vs, Wave wv, uint32
     if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
 }
 
+// An unoccluded shadow ray's emission goes to its path's radiance.
+struct Unoccluded {
+    const float4* emission;
+    float4* state;
+    __device__ __forceinline__ void add(uint32_t ray) const
+    {
+        const float4 c = emission[ray];
+        float4* st = state + 2 * (size_t)__float_as_uint(c.w);
+        const float4 a = *st;
+        *st = make_float4(__fadd_rn(a.x, c.x), __fadd_rn(a.y, c.y), __fadd_rn(a.z, c.z), a.w);
+    }
+    __device__ __forceinline__ void hit(uint32_t, float, float, float, float) const {}
+    __device__ __forceinline__ void done(uint32_t ray, const WideState& s) const
+    {
+        if (s.t != kWideFound) add(ray);
+    }
+    __device__ __forceinline__ uint32_t found(uint32_t) const { return CPT_INVALID_INDEX; }
+};
+
 // Shadow rays of next-event estimation: any-hit up to each ray's far limit; an
 // unoccluded ray adds its emission to its path's radiance (one shadow ray per
 // path and vertex, so no two threads add to the same path).
@@ -655,17 +672,10 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_occlude
                                                           uint32_t* __restrict__ pool, float4* __restrict__ state,
                                                           uint32_t* __restrict__ status)
 {
-    __shared__ __align__(16) uint32_t s_stack[kSmemStack * kExtendBlock];
+    __shared__ __align__(16) uint32_t s_stack[(kWide ? 2 * kWideSmemStack : kSmemStack) * kExtendBlock];
     const uint32_t n = *count;
     bool overflow = false;
     uint32_t nn = 0, nt = 0;
-    auto add_unoccluded = [&](uint32_t ray, const Hit& best) {
-        if (best.tri != CPT_INVALID_INDEX) return;
-        const float4 c = emission[ray];
-        float4* st = state + 2 * (size_t)__float_as_uint(c.w);
-        const float4 a = *st;
-        *st = make_float4(__fadd_rn(a.x, c.x), __fadd_rn(a.y, c.y), __fadd_rn(a.z, c.z), a.w);
-    };
     if constexpr (kWide) {
         auto wide_of = [&](uint32_t vi, uint32_t& mv, const float4*& tr) -> const float4* {
             const uint32_t v = kOneView ? 0u : vi;
@@ -673,9 +683,9 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_occlude
             tr = vs.v[v].wide_tris;
             return vs.v[v].wide_nodes;
         };
-        persistent_trace_wide<true, kExtendBlock, false, kExtendSteps, true>(
+        persistent_trace_wide<true, kExtendBlock, false, kExtendSteps, true, true>(
             wide_of, rays, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, nullptr,
-            [&](uint32_t ray, const WideState& s) { add_unoccluded(ray, s.best); });
+            Unoccluded{emission, state});
         if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
         return;
     }
@@ -691,7 +701,9 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_occlude
     };
     persistent_trace<true, kExtendBlock, false, kExtendSteps, true>(
         view_nodes, rays, n, pool, s_stack + threadIdx.x, overflow, nn, nt, nullptr,
-        [&](uint32_t ray, const TraceState& s) { add_unoccluded(ray, s.best); });
+        [&](uint32_t ray, const TraceState& s) {
+            if (s.best.tri == CPT_INVALID_INDEX) Unoccluded{emission, state}.add(ray);
+        });
     if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
 }
 
@@ -1103,7 +1115,8 @@ int render_views(const Views& vs, bool any_lights, const cpt_bbox* sort_root, co
                          st>>>(wl, vs, L.queue[0], L.counts, rs.state);
         }
         CPT_LAUNCH_CHECK();
-        const int ext_blocks = std::min<int>((int)((paths + kExtendBlock - 1) / kExtendBlock), sms * per_sm);
+        const uint32_t block_rays = wide ? (uint32_t)(kWideMinLanes * kExtendBlock / 32) : (uint32_t)kExtendBlock;
+        const int ext_blocks = std::min<int>((int)((paths + block_rays - 1) / block_rays), sms * per_sm);
         const int shade_blocks = std::min<int>((int)((paths + kShadeBlock - 1) / kShadeBlock), sms * 16);
         for (uint32_t b = 0; b <= params->bounces; ++b) {
             const float4* qin = L.queue[b & 1];

@@ -317,7 +317,9 @@ __device__ __forceinline__ Hit traverse(const float4* __restrict__ nodes, f3 o, 
 // taken, visits the next node of the node group (the rest of the group goes on the
 // stack; the node's triangle group queues behind), or pops a group. The triangle test
 // is tri_test on the binary leaf slot's words, so a hit's t, u, v are unchanged.
-constexpr int kWideSmemStack = 16;  // stack entries (2 words) per thread in shared memory
+// stack entries (2 words) per thread in shared memory (8, 12 and 16 run alike; with the words
+// that share a launch's last rays, 8 blocks of 128 threads stay within a 164 KB split)
+constexpr int kWideSmemStack = 15;
 constexpr float kWideGrow = 1.0f + 1.0f / 262144.0f;  // relative slack of a wide child's box test
 // Records a leaf slot holds at most: binary subtrees of up to this many leaves become one
 // leaf slot of their parent wide node instead of a wide node of their own; a wide tree
@@ -356,14 +358,15 @@ constexpr float kWideFarInv = 1099511627776.0f;  // 2^40: 1/d of a zero directio
 #endif
 constexpr int kWideTriBatch = CPT_WIDE_TRI_BATCH;
 
+constexpr float kWideFound = -1.0f;  // an any-hit ray's t once it is occluded
+
 struct WideState {
     const float4* nodes;
     const float4* tris;
     uint32_t max_visits;  // wide node fetches allowed (the wide tree's node capacity)
-    uint32_t tri_cap;     // triangle records
     f3 o, d, dinv;
     uint32_t oct;         // direction sign bits (x: 1, y: 2, z: 4)
-    Hit best;
+    float t;              // nearest hit so far (kAny: kWideFound once there is one)
     uint32_t cbase, gbits;  // node group: first child; bits 0-7 hit slots in visit order, 8-15 internal mask
     uint32_t tbase, tbits;  // triangle group: first record; records to test (kWideRecBits), leaf mask << 24
     uint32_t tbase2, tbits2;  // a second triangle group, queued behind the first
@@ -378,18 +381,13 @@ __device__ __forceinline__ void wide_init(WideState& s, const float4* nodes, con
     s.nodes = nodes;
     s.tris = tris;
     s.max_visits = max_visits;
-    s.tri_cap = kWideRecordLayers * (max_visits + 1);
     s.o = o;
     s.d = d;
     const float ix = __frcp_rn(d.x), iy = __frcp_rn(d.y), iz = __frcp_rn(d.z);
     s.dinv = mk3(isfinite(ix) ? ix : copysignf(kWideFarInv, d.x), isfinite(iy) ? iy : copysignf(kWideFarInv, d.y),
                  isfinite(iz) ? iz : copysignf(kWideFarInv, d.z));
     s.oct = (s.dinv.x < 0.f ? 1u : 0u) | (s.dinv.y < 0.f ? 2u : 0u) | (s.dinv.z < 0.f ? 4u : 0u);
-
-    s.best.t = FLT_MAX;
-    s.best.u = 0.f;
-    s.best.v = 0.f;
-    s.best.tri = CPT_INVALID_INDEX;
+    s.t = FLT_MAX;
     s.cbase = 0;  // the root, wide node 0: the one internal slot (0) of a virtual parent, visited first
     s.gbits = (1u << s.oct) | (1u << 8);
     s.tbase = 0;
@@ -479,7 +477,7 @@ __device__ __forceinline__ uint32_t wide_child_hits(const WideState& s, float4 n
     const uint32_t px0 = (oct & 1u) ? 0x4041u : 0x4140u, py0 = (oct & 2u) ? 0x4041u : 0x4140u,
                    pz0 = (oct & 4u) ? 0x4041u : 0x4140u;
     const uint32_t sel[2][3] = {{px0, py0, pz0}, {px0 + 0x0202u, py0 + 0x0202u, pz0 + 0x0202u}};
-    const float tlim = s.best.t;
+    const float tlim = s.t;
     uint32_t hm = 0;
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {  // two children at a time
@@ -506,10 +504,14 @@ __device__ __forceinline__ uint32_t wide_child_hits(const WideState& s, float4 n
 
 // One step; returns true when the ray is finished.
 // perm: xor_permute8 as a table in shared memory, byte oct * 256 + x (wide_perm_table).
-template <bool kAny, int kBlock, bool kStats>
+// bot: the lowest stack entry still the lane's own (above 0 once others have been given
+// away from the bottom; see wide_tail).
+// hit(t, u, v, triangle): a nearer hit than any before (kAny: the hit). tie(triangle): a
+// triangle at exactly the nearest hit's distance.
+template <bool kAny, int kBlock, bool kStats, typename OnHit, typename OnTie>
 __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* spill, bool& overflow,
-                                          uint32_t& n_nodes, uint32_t& n_tris, const uint8_t* perm,
-                                          bool test_tri = true)
+                                          uint32_t& n_nodes, uint32_t& n_tris, const uint8_t* perm, OnHit hit,
+                                          OnTie tie, bool test_tri = true, int bot = 0)
 {
     if (test_tri && (s.tbits & kWideRecBits)) {
         // the lowest record bit, 8j + slot (the leaf mask lies above): record j * L + rank
@@ -518,19 +520,19 @@ __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* 
         const uint32_t below = (s.tbits ^ t1) >> 1;
         const uint32_t idx = s.tbase + __popc(((s.tbits >> 24) * 0x010101u) & below);
         s.tbits &= t1;
-        if (idx >= s.tri_cap) { overflow = true; return true; }
+        if (idx >= kWideRecordLayers * (s.max_visits + 1)) { overflow = true; return true; }
         const float4 a = __ldg(s.tris + 3 * (size_t)idx), b = __ldg(s.tris + 3 * (size_t)idx + 1),
                      c = __ldg(s.tris + 3 * (size_t)idx + 2);
         const float w[10] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, c.x, c.y, c.z};
         float u, v;
         const float t = tri_test(s.o, s.d, w, u, v);
         if (kStats) { ++n_tris; ++s.tests; }
-        if (t < s.best.t) {
-            s.best.t = t;
-            s.best.u = u;
-            s.best.v = v;
-            s.best.tri = __float_as_uint(a.w);
+        if (t < s.t) {
+            s.t = kAny ? kWideFound : t;
+            hit(t, u, v, a.w);
             if (kAny) return true;
+        } else if (t == s.t) {
+            tie(a.w);
         }
         if (!(s.tbits & kWideRecBits) && (s.tbits2 & kWideRecBits)) {  // the queued groups move up
             s.tbase = s.tbase2;
@@ -542,7 +544,7 @@ __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* 
         if (s.tbits3 & kWideRecBits) return false;  // every group slot pending: no node visit this step
     }
     if (!(s.gbits & 0xFFu)) {
-        if (s.sp == 0) return !(s.tbits & kWideRecBits);  // done once the last triangles are tested
+        if (s.sp == bot) return !(s.tbits & kWideRecBits);  // done once the last triangles are tested
         const uint2 g = wide_pop<kBlock>(smem_col, spill, s.sp);
         s.cbase = g.x;
         s.gbits = g.y;
@@ -647,14 +649,246 @@ __device__ __forceinline__ void persistent_trace(NodesOf nodes_of, const float4*
     }
 }
 
+// Whether the warp tests triangles in this step: when enough lanes have some pending, or
+// when a lane must (every group slot taken, or no node left to visit).
+__device__ __forceinline__ bool wide_test_now(const WideState& s, bool live)
+{
+    if (!kWideTriBatch) return true;
+    const bool want = live && (s.tbits & kWideRecBits);
+    const bool must = want && ((s.tbits3 & kWideRecBits) || (!(s.gbits & 0xFFu) && s.sp == 0));
+    const unsigned bw = __ballot_sync(0xFFFFFFFFu, want);
+    return __ballot_sync(0xFFFFFFFFu, must) != 0u || __popc(bw) >= kWideTriBatch;
+}
+
+// Lanes of a warp that take rays from the pool of n: all, or, where the grid has more
+// lanes than there are rays, the grid's even share, so that every warp has rays and the
+// lanes left over help with them (wide_tail); at least kWideMinLanes of them, because a
+// warp's step costs the same for one ray as for eight (1.3 M-triangle hairball scene, a
+// launch of 1,000 / 10,000 / 60,000 rays: 256 / 350 / 488 us with 1, 223 / 315 / 486 with
+// 4, 186 / 291 / 489 with 8, 237 / 324 / 492 with 16, 263 / 375 / 504 with all 32; without
+// helpers 387 / 739 / 1,231 us). Launches size their grids by it.
+constexpr uint32_t kWideMinLanes = 8;
+__device__ __forceinline__ uint32_t wide_ray_lanes(uint32_t n)
+{
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    return min(32u, max(kWideMinLanes, n / warps + (n % warps != 0u)));
+}
+
+// The end of a launch. Once the ray pool is empty a warp's lanes run out of rays one by
+// one, and the launch lasts as long as its slowest rays: thousands of node visits one
+// after the other, each a dependent L2 access, against about 65 on average (hairball
+// scenes), with the rest of the chip idle. So once kWideTailLanes lanes or fewer are left,
+// the idle lanes take work from the busy ones: an idle lane copies a busy lane's ray and
+// takes the bottom entry of its stack (the node group nearest the root, so the largest
+// piece of work) to traverse with a stack of its own. All lanes at work on a ray share its
+// nearest distance (t, indexed by the ray's lane), so each prunes with what any of them has
+// found. A ray is finished when its own lane and all its helpers are.
+//
+// Measured (before -> after): C1's frame 1,008 -> 808 us, a 1280x720 one-sample frame with
+// shadow rays 6.1 -> 3.6 ms, one million incoherent rays 3.7 -> 3.0 ms, 10,000 of them 740 ->
+// 250 us, C2's 16-sample frame 94.9 -> 93.3 ms. Thresholds 8 / 12 / 16 lanes: 809 / 789 / 786
+// us and 4.52 / 4.37 / 4.37 ms on the first two in an earlier form; 28 and 31 lose (helpers
+// visit nodes that a nearer hit would have culled). It is a function of its own, called with
+// a copy of the state, because the loop before it has no register to spare: inlined, or with
+// the state live across the loop's end, C2 ran 5 to 8 % slower. For the same reason a hit is
+// written when it is found instead of carried (u, v, triangle) to the ray's end.
+//
+// The hit is the one that a lane finds alone: a child box is wide enough that no order of
+// visits loses a hit (the binary trees' boxes are not, and their traversal keeps the
+// reference's order), and a ray that meets two triangles at exactly its nearest distance,
+// of which a lane alone reports the one it visits first, is traced anew by its own lane
+// alone (two or three rays of a million; from the start, since a split triangle may be met
+// first through the box of a piece that does not hold the hit). Every iteration each working
+// lane consumes a node, a stack entry or a triangle, as in the main loop; a helper goes on
+// counting its donor's node visits and the iterations are limited, so that a corrupt tree
+// ends in an overflow report.
+constexpr int kWideTailLanes = 12;
+struct WideTail {  // per warp, in shared memory
+    int t[32];          // float bits of the ray's nearest distance (as int: -0 and kWideFound sort lowest)
+    uint32_t tri[32];   // the triangle there
+    uint32_t info[32];  // byte 0: helpers at work; byte 1 (of word r): the r-th lane with a stack entry to give;
+                        // bit 31: another triangle lies at exactly the nearest distance
+};
+
+template <bool kAny, int kBlock, typename Sink>
+__device__ __noinline__ bool wide_tail(WideState s, uint32_t ray, uint2* smem_col, uint2* spill, const uint8_t* perm,
+                                       WideTail& w, Sink sink)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    uint32_t owner = lane;
+    uint32_t target = ray;  // the ray this lane works for
+    bool work = ray != CPT_INVALID_INDEX;
+    bool overflow = false;
+    int bot = 0;
+    uint32_t nn = 0, nt = 0;
+    constexpr uint32_t kTie = 0x80000000u;
+    bool alone = false;  // a ray traced anew: its lane gives nothing away
+    // more steps than the longest valid traversal takes: its nodes and their records
+    uint32_t limit = __reduce_max_sync(0xFFFFFFFFu, work ? s.max_visits : 0u);
+    limit = limit < (1u << 26) ? 32u * limit + 1024u : 0x80000000u;
+    bool share = false;  // until kWideTailLanes lanes are left, each traces its own ray as in the main loop
+#pragma unroll 1
+    for (uint32_t iter = 0;; ++iter) {
+        const unsigned wm = __ballot_sync(0xFFFFFFFFu, work);
+        if (wm == 0u) break;
+        bool test_tri = true;
+        if (!share) {
+            if (__popc(wm) <= kWideTailLanes) {
+                share = true;
+                w.t[lane] = __float_as_int(s.t);
+                w.info[lane] = 0;
+                if (!kAny && work && s.t < FLT_MAX) w.tri[lane] = sink.found(ray);
+                __syncwarp();
+            } else {
+                test_tri = wide_test_now(s, work);
+            }
+        }
+        const bool idle = !work && ray == CPT_INVALID_INDEX;  // (a ray's own lane waits for its helpers)
+        const bool give = work && !alone && s.sp > bot && bot < kWideSmemStack;
+        const unsigned im = __ballot_sync(0xFFFFFFFFu, idle), dm = __ballot_sync(0xFFFFFFFFu, give);
+        if (share && im && dm) {
+            if (give) reinterpret_cast<uint8_t*>(&w.info[__popc(dm & lt_mask)])[1] = (uint8_t)lane;
+            __syncwarp();
+            const uint32_t r = (uint32_t)__popc(im & lt_mask);
+            const bool take = idle && r < (uint32_t)__popc(dm);
+            const int src = take ? (int)((w.info[r] >> 8) & 31u) : (int)lane;
+            __syncwarp();
+            const float ox = __shfl_sync(0xFFFFFFFFu, s.o.x, src), oy = __shfl_sync(0xFFFFFFFFu, s.o.y, src),
+                        oz = __shfl_sync(0xFFFFFFFFu, s.o.z, src);
+            const float dx = __shfl_sync(0xFFFFFFFFu, s.d.x, src), dy = __shfl_sync(0xFFFFFFFFu, s.d.y, src),
+                        dz = __shfl_sync(0xFFFFFFFFu, s.d.z, src);
+            const unsigned long long pn =
+                __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(s.nodes), src);
+            const unsigned long long pt = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(s.tris), src);
+            const uint32_t mv = __shfl_sync(0xFFFFFFFFu, s.max_visits, src);
+            const float bt = __shfl_sync(0xFFFFFFFFu, s.t, src);
+            const uint32_t ow = __shfl_sync(0xFFFFFFFFu, owner, src), tg = __shfl_sync(0xFFFFFFFFu, target, src);
+            const int sb = __shfl_sync(0xFFFFFFFFu, bot, src);
+            const uint32_t vis = __shfl_sync(0xFFFFFFFFu, s.visits, src);  // (so a cycle uses up its limit)
+            if (take) {
+                wide_init(s, reinterpret_cast<const float4*>(pn), reinterpret_cast<const float4*>(pt), mv,
+                          mk3(ox, oy, oz), mk3(dx, dy, dz));
+                const uint2 g = (smem_col + (src - (int)lane))[sb * kBlock];
+                s.cbase = g.x;
+                s.gbits = g.y;
+                s.t = bt;
+                s.visits = vis;
+                owner = ow;
+                target = tg;
+                bot = 0;
+                work = true;
+                alone = false;
+                atomicAdd(&w.info[ow], 1u);
+            }
+            if (give && __popc(dm & lt_mask) < __popc(im)) {  // the bottom entry is the taker's now
+                ++bot;
+                if (bot == s.sp) bot = s.sp = 0;
+            }
+            __syncwarp();
+        }
+        bool fin = false, found = false;
+        float hu = 0.f, hv = 0.f, htri = 0.f, ht = 0.f;
+        if (work) {
+            fin = wide_step<kAny, kBlock, false>(
+                s, smem_col, spill, overflow, nn, nt, perm,
+                [&](float t, float u, float v, float tri) {
+                    if (share) {
+                        found = true;
+                        ht = t; hu = u; hv = v; htri = tri;
+                    } else {
+                        sink.hit(ray, t, u, v, tri);
+                    }
+                },
+                [&](float tri) {
+                    if (!kAny && share && s.t < FLT_MAX && w.tri[owner] != __float_as_uint(tri))
+                        atomicOr(&w.info[owner], kTie);
+                },
+                test_tri, bot);
+            if (found) atomicMin(&w.t[owner], __float_as_int(s.t));
+            if (iter >= limit) { overflow = true; fin = true; }
+        }
+        if (!share) {
+            if (fin) {
+                sink.done(ray, s);
+                work = false;
+                ray = CPT_INVALID_INDEX;
+            }
+            continue;
+        }
+        __syncwarp();
+        if (work || ray != CPT_INVALID_INDEX) {
+            const float near = __int_as_float(*reinterpret_cast<volatile int*>(&w.t[owner]));
+            found = found && near == s.t;
+            s.t = near;
+            if (kAny && near == kWideFound) fin = work;
+        }
+        // nearer hits are reported one lane after the other; of several at one distance the
+        // first is, and the tie noted
+        for (unsigned hm = __ballot_sync(0xFFFFFFFFu, found), seen = 0; hm; hm &= hm - 1u) {
+            const int l = __ffs(hm) - 1;
+            const uint32_t ow = __shfl_sync(0xFFFFFFFFu, owner, l);
+            if ((int)lane == l) {
+                if ((seen >> ow) & 1u) {
+                    if (!kAny && w.tri[ow] != __float_as_uint(htri)) atomicOr(&w.info[ow], kTie);
+                } else {
+                    if (!kAny) {
+                        w.tri[ow] = __float_as_uint(htri);
+                        atomicAnd(&w.info[ow], ~kTie);
+                    }
+                    sink.hit(target, ht, hu, hv, htri);
+                }
+            }
+            seen |= 1u << ow;
+            __syncwarp();
+        }
+        if (fin) {
+            work = false;
+            if (owner != lane) atomicSub(&w.info[owner], 1u);
+        }
+        __syncwarp();
+        if (ray != CPT_INVALID_INDEX && !work && (w.info[lane] & 0xFFu) == 0u) {
+            if (!kAny && (w.info[lane] & kTie) && !alone) {
+                const float4* nodes = s.nodes;
+                wide_init(s, nodes, s.tris, s.max_visits, s.o, s.d);
+                bot = 0;
+                alone = work = true;
+                w.t[lane] = __float_as_int(s.t);
+            } else {
+                sink.done(ray, s);
+                ray = CPT_INVALID_INDEX;
+            }
+        }
+        __syncwarp();
+    }
+    return overflow;
+}
+
+// Closest hits written to hits[ray] = (t, u, v, triangle) as they are found.
+struct WideHits {
+    float4* hits;
+    __device__ __forceinline__ void hit(uint32_t ray, float t, float u, float v, float tri) const
+    {
+        hits[ray] = make_float4(t, u, v, tri);
+    }
+    __device__ __forceinline__ void done(uint32_t ray, const WideState& s) const
+    {
+        if (s.t == FLT_MAX) hits[ray] = make_float4(FLT_MAX, 0.f, 0.f, __uint_as_float(CPT_INVALID_INDEX));
+    }
+    __device__ __forceinline__ uint32_t found(uint32_t ray) const { return __float_as_uint(hits[ray].w); }
+};
+
 // persistent_trace over wide BVHs: wide_of(w, max_visits, tris) returns the wide
 // node array, its node capacity and its triangle records for the word w of the
 // direction's .w. Same refill rule and far-limit convention as persistent_trace.
-template <bool kAny, int kBlock, bool kStats, int kSteps, bool kTmax, typename WideOf, typename Done>
+// sink.hit(ray, t, u, v, triangle) is called for every nearer hit, sink.done(ray, state) once
+// at the ray's end; sink.found(ray) is the triangle of the last hit given to sink.hit. kTail:
+// the launch's end shares rays among lanes (wide_tail).
+template <bool kAny, int kBlock, bool kStats, int kSteps, bool kTmax, bool kTail, typename WideOf, typename Sink>
 __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const float4* __restrict__ rays, uint32_t n,
                                                       uint32_t* __restrict__ pool, uint2* smem_col, bool& overflow,
                                                       uint32_t& n_nodes, uint32_t& n_tris,
-                                                      const uint32_t* __restrict__ order, Done done,
+                                                      const uint32_t* __restrict__ order, Sink sink,
                                                       uint32_t refill = 0)
 {
     const uint32_t refill_below = refill ? refill : (uint32_t)kWideRefillLanes;
@@ -666,16 +900,20 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
     WideState s;
     uint32_t ray = CPT_INVALID_INDEX;
     bool drained = false;
+    static_assert(!kTail || kAny || !kTmax, "a ray traced anew starts unbounded");
+    const uint32_t lanes = kTail ? wide_ray_lanes(n) : 32u;
+    // one grab per warp takes all the rays
+    const bool once = kTail && n <= lanes * (gridDim.x * (blockDim.x / 32u));
     for (;;) {
         if (!drained) {
-            const bool idle = ray == CPT_INVALID_INDEX;
+            const bool idle = ray == CPT_INVALID_INDEX && (!kTail || lane < lanes);
             const unsigned m = __ballot_sync(0xFFFFFFFFu, idle);
             if (m) {
                 const int leader = __ffs(m) - 1;
                 uint32_t base = 0;
                 if ((int)lane == leader) base = atomicAdd(pool, (uint32_t)__popc(m));
                 base = __shfl_sync(0xFFFFFFFFu, base, leader);
-                if (base + (uint32_t)__popc(m) >= n) drained = true;
+                if (base + (uint32_t)__popc(m) >= n || once) drained = true;
                 if (idle) {
                     const uint32_t r = base + (uint32_t)__popc(m & lt_mask);
                     if (r < n) {
@@ -686,7 +924,7 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
                             const float4* tris;
                             const float4* nodes = wide_of(__float_as_uint(rd.w), mv, tris);
                             wide_init(s, nodes, tris, mv, mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z));
-                            if (kTmax) s.best.t = ro.w;
+                            if (kTmax) s.t = ro.w;
                         } else {  // a ray order left void by a failed sort
                             overflow = true;
                             ray = CPT_INVALID_INDEX;
@@ -695,30 +933,29 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
                 }
             }
         }
+        if (kTail && drained) break;
         if (__ballot_sync(0xFFFFFFFFu, ray != CPT_INVALID_INDEX) == 0) break;
 #pragma unroll 1
         for (int k = 1;; ++k) {
-            bool test_tri = true;
-            if (kWideTriBatch) {
-                // the warp tests triangles when enough lanes have some pending, or when a lane
-                // must (every group slot taken, or no node left to visit)
-                const bool live = ray != CPT_INVALID_INDEX;
-                const bool want = live && (s.tbits & kWideRecBits);
-                const bool must = want && ((s.tbits3 & kWideRecBits) || (!(s.gbits & 0xFFu) && s.sp == 0));
-                const unsigned bw = __ballot_sync(0xFFFFFFFFu, want);
-                test_tri = __ballot_sync(0xFFFFFFFFu, must) != 0u || __popc(bw) >= kWideTriBatch;
-            }
+            const bool test_tri = wide_test_now(s, ray != CPT_INVALID_INDEX);
             if (ray != CPT_INVALID_INDEX &&
-                wide_step<kAny, kBlock, kStats>(s, smem_col, spill, overflow, n_nodes, n_tris, s_perm, test_tri)) {
-                done(ray, s);
+                wide_step<kAny, kBlock, kStats>(
+                    s, smem_col, spill, overflow, n_nodes, n_tris, s_perm,
+                    [&](float t, float u, float v, float tri) { sink.hit(ray, t, u, v, tri); }, [](float) {}, test_tri)) {
+                sink.done(ray, s);
                 ray = CPT_INVALID_INDEX;
             }
             const unsigned live = __ballot_sync(0xFFFFFFFFu, ray != CPT_INVALID_INDEX);
             if (live == 0) break;
-            if (!drained && ((uint32_t)__popc(live) < refill_below || k >= kSteps)) break;
+            if ((kTail || !drained) && ((uint32_t)__popc(live) < refill_below || k >= kSteps)) break;
         }
     }
+    if (kTail && __ballot_sync(0xFFFFFFFFu, ray != CPT_INVALID_INDEX) != 0u) {
+        __shared__ WideTail s_tail[kBlock / 32];
+        overflow |= wide_tail<kAny, kBlock>(s, ray, smem_col, spill, s_perm, s_tail[threadIdx.x >> 5], sink);
+    }
 }
+
 
 // persistent_trace of unbounded rays whose hit goes to hits[i] = (t, u, v, triangle).
 // ray_stats (nullable, with kStats): per ray (node fetches, triangle tests).
