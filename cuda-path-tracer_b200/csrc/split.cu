@@ -508,7 +508,6 @@ constexpr int kTreeletBlock = 128;
 constexpr int kTreeletWarps = kTreeletBlock / 32;
 constexpr int kTreeletLeaves = 7;
 constexpr int kTreeletSubsets = 1 << kTreeletLeaves;
-constexpr int kTreeletPairs = 966;  // sum over k = 2..7 of C(7, k) (2^(k-1) - 1)
 #ifndef CPT_TREELET_ROUNDS
 #define CPT_TREELET_ROUNDS 1
 #endif
@@ -522,21 +521,6 @@ constexpr int kTreeletRounds = CPT_TREELET_ROUNDS;
 constexpr int kTreeletGamma = CPT_TREELET_GAMMA;
 constexpr int kTreeletMaxLevels = 1024;
 
-// Index of the first (subset, split) pair of the subsets of k leaves (k = 2..7;
-// k = 8 gives the total).
-__device__ __forceinline__ int treelet_class_start(int k)
-{
-    switch (k) {
-    case 2: return 0;
-    case 3: return 21;
-    case 4: return 126;
-    case 5: return 371;
-    case 6: return 686;
-    case 7: return 903;
-    default: return kTreeletPairs;
-    }
-}
-
 // Half the surface area of a box (lo xyz, hi xyz), rounded alike on every run.
 __device__ __forceinline__ float half_area(const float* b)
 {
@@ -544,255 +528,340 @@ __device__ __forceinline__ float half_area(const float* b)
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dy), __fmul_rn(dy, dz)), __fmul_rn(dz, dx));
 }
 
-// A treelet as formed: its leaves and internal nodes.
-struct TreeletForm {
+// A warp's treelet. Lane k stands for treelet leaf k while it is formed. c comes first, at a
+// multiple of its 512 B in shared memory: a subset's byte offset is then or-ed into its address.
+struct alignas(512) TreeletWarp {
+    float c[kTreeletSubsets];            // least cost over a subset (its area until its size class is done)
     float box[kTreeletLeaves][6];
-    uint32_t id[kTreeletLeaves];      // internal node index, or piece position for a leaf
+    float slot[kTreeletLeaves][10];      // the leaves' 40-B child slots, read before any rewrite
+    uint32_t id[kTreeletLeaves];         // internal node index, or piece position for a leaf
     uint32_t height[kTreeletLeaves];
     uint32_t size[kTreeletLeaves];
-    uint32_t from[kTreeletLeaves];    // parent * 2 + side: the record slot holding the leaf
     uint32_t inode[kTreeletLeaves - 1];  // the treelet's internal nodes, [0] = its root
-    uint32_t internal_mask;           // bit k: treelet leaf k is an internal node
-    uint32_t m;                       // treelet leaves (0: bad index met)
-    float old_cost;                   // summed area of the treelet's internal nodes
+    uint8_t split[kTreeletSubsets];      // and the part of it with its lowest leaf
+    // the new topology: node j covers subset sub[j], its children are treelet leaf k (< 8) or node 8 + j
+    uint8_t sub[kTreeletLeaves - 1], child[kTreeletLeaves - 1][2], node_depth[kTreeletLeaves - 1];
+    uint8_t leaf_depth[kTreeletLeaves];
 };
 
-struct TreeletWarp {
-    TreeletForm form;
-    float c[kTreeletSubsets];         // least cost over a subset (its area until its size class is done)
-    float slot[kTreeletLeaves][10];   // the leaves' 40-B child slots, read before any rewrite
-    uint8_t split[kTreeletSubsets];
+// The subsets of 7 leaves by size: 21 of 2 (from 0), 35 of 3 (21), 35 of 4 (56), 21 of 5 (91),
+// 7 of 6 (112) and the whole (119).
+__constant__ uint8_t kTreeletOrder[120] = {
+    3, 5, 6, 9, 10, 12, 17, 18, 20, 24, 33, 34, 36, 40, 48, 65, 66, 68, 72, 80, 96,
+    7, 11, 13, 14, 19, 21, 22, 25, 26, 28, 35, 37, 38, 41, 42, 44, 49, 50, 52, 56, 67, 69, 70, 73, 74, 76, 81, 82, 84, 88,
+    97, 98, 100, 104, 112,
+    15, 23, 27, 29, 30, 39, 43, 45, 46, 51, 53, 54, 57, 58, 60, 71, 75, 77, 78, 83, 85, 86, 89, 90, 92, 99, 101, 102, 105,
+    106, 108, 113, 114, 116, 120,
+    31, 47, 55, 59, 61, 62, 79, 87, 91, 93, 94, 103, 107, 109, 110, 115, 117, 118, 121, 122, 124,
+    63, 95, 111, 119, 123, 125, 126, 127};
+
+// What treelet_form leaves in registers, the same in every lane.
+struct TreeletForm {
+    uint32_t m;              // treelet leaves (0: bad index met)
+    uint32_t internal_mask;  // bit k: treelet leaf k is an internal node
+    float old_cost;          // summed area of the treelet's internal nodes
 };
 
-// Treelet leaves k0 and k1 := the two children of internal node q. False on an out-of-range index.
-__device__ bool treelet_take_children(const float* __restrict__ nodes, const float4* __restrict__ leaf_boxes,
-                                      const uint2* __restrict__ info, uint32_t n, uint32_t q, int k0, int k1,
-                                      TreeletForm& f)
+// Forms the treelet rooted at internal node r (the whole warp): one coalesced load per opened
+// node brings both child slots; the lanes of the two new treelet leaves fetch what hangs on
+// them (boxes of pieces, sizes and heights of nodes).
+__device__ __forceinline__ TreeletForm treelet_form(const float* __restrict__ nodes,
+                                                    const float4* __restrict__ leaf_boxes,
+                                                    const uint2* __restrict__ info, uint32_t n, uint32_t r,
+                                                    TreeletWarp& w, uint32_t* __restrict__ status)
 {
-    const float* rec = nodes + 24 * (size_t)q;
-    const float4 meta = __ldcg(reinterpret_cast<const float4*>(rec + 20));
-    const uint32_t word = __float_as_uint(meta.x);
-    const uint32_t ids[2] = {word >> 2, __float_as_uint(meta.y)};
-    for (int side = 0; side < 2; ++side) {
-        const int k = side ? k1 : k0;
-        const bool internal = (word >> side) & 1u;
-        const uint32_t id = ids[side];
-        if (internal ? id >= n - 1 : id >= n) return false;
-        if (internal) {  // an internal child's slot starts with its box
-            const float2* sp = reinterpret_cast<const float2*>(rec + 10 * side);
-            const float2 a = __ldcg(sp), b = __ldcg(sp + 1), c = __ldcg(sp + 2);
-            f.box[k][0] = a.x; f.box[k][1] = a.y; f.box[k][2] = b.x;
-            f.box[k][3] = b.y; f.box[k][4] = c.x; f.box[k][5] = c.y;
-            const uint2 g = __ldcg(info + id);
-            f.size[k] = g.x;
-            f.height[k] = g.y;
-            f.internal_mask |= 1u << k;
-        } else {
-            const float4 lo = leaf_boxes[2 * (size_t)id], hi = leaf_boxes[2 * (size_t)id + 1];
-            f.box[k][0] = lo.x; f.box[k][1] = lo.y; f.box[k][2] = lo.z;
-            f.box[k][3] = hi.x; f.box[k][4] = hi.y; f.box[k][5] = hi.z;
-            f.size[k] = 1;
-            f.height[k] = 0;
-            f.internal_mask &= ~(1u << k);
+    const uint32_t lane = threadIdx.x & 31u;
+    TreeletForm f;
+    f.old_cost = 0.f;
+    uint32_t m = 0, q = r, k0 = 0, id = 0, size = 0, height = 0;
+    uint32_t cand = 0;  // an internal leaf's area as bits + 1
+    bool internal = false, ok = true;
+    __syncwarp();  // the last treelet's readers are done
+    for (uint32_t ni = 0;; ++ni) {
+        const uint32_t k1 = m ? m : 1u;
+        if (lane == 0) w.inode[ni] = q;
+        // words 0-9 the left slot, 10-19 the right, 20 the Node word, 21 the right child
+        const float wd = lane < 22u ? __ldcg(nodes + 24 * (size_t)q + lane) : 0.f;
+        const uint32_t word = __shfl_sync(0xFFFFFFFFu, __float_as_uint(wd), 20);
+        const uint32_t right = __shfl_sync(0xFFFFFFFFu, __float_as_uint(wd), 21);
+        const uint32_t side = lane >= 10u ? 1u : 0u, at = lane - 10u * side;
+        const bool side_internal = (word >> side) & 1u;
+        const uint32_t side_id = side ? right : word >> 2;
+        ok = ok && !__any_sync(0xFFFFFFFFu, side_internal ? side_id >= n - 1 : side_id >= n);
+        if (!ok) break;
+        if (lane < 20u) {
+            const uint32_t k = side ? k1 : k0;
+            w.slot[k][at] = wd;
+            if (at < 6u)  // an internal child's slot starts with its box
+                w.box[k][at] = side_internal
+                                   ? wd
+                                   : reinterpret_cast<const float*>(leaf_boxes)[8 * (size_t)side_id + at + (at >= 3u)];
         }
-        f.id[k] = id;
-        f.from[k] = 2u * q + (uint32_t)side;
+        if (lane == k0 || lane == k1) {
+            const bool rhs = lane == k1;
+            internal = (word >> (rhs ? 1 : 0)) & 1u;
+            id = rhs ? right : word >> 2;
+            const uint2 g = internal ? __ldcg(info + id) : make_uint2(1u, 0u);
+            size = g.x;
+            height = g.y;
+        }
+        __syncwarp();
+        if (lane == k0 || lane == k1) {
+            const float a = half_area(w.box[lane]);
+            cand = internal && a >= 0.f ? __float_as_uint(a) + 1u : 0u;
+        }
+        if (m == 0) {
+            float rb[6];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                rb[a] = fminf(w.box[0][a], w.box[1][a]);
+                rb[3 + a] = fmaxf(w.box[0][3 + a], w.box[1][3 + a]);
+            }
+            f.old_cost = half_area(rb);
+        }
+        m = k1 + 1u;
+        if (m == (uint32_t)kTreeletLeaves) break;
+        const uint32_t mx = __reduce_max_sync(0xFFFFFFFFu, lane < m ? cand : 0u);
+        if (mx == 0u) break;
+        k0 = (uint32_t)__ffs(__ballot_sync(0xFFFFFFFFu, lane < m && cand == mx)) - 1u;  // the first of largest area
+        q = __shfl_sync(0xFFFFFFFFu, id, k0);
+        f.old_cost = __fadd_rn(f.old_cost, __uint_as_float(mx - 1u));
     }
-    return true;
+    if (!ok && lane == 0) atomicOr(status, CPT_STATUS_BAD_INDEX);
+    f.m = ok ? m : 0u;
+    f.internal_mask = __ballot_sync(0xFFFFFFFFu, lane < m && internal);
+    if (lane < m) {
+        w.id[lane] = id;
+        w.size[lane] = size;
+        w.height[lane] = height;
+    }
+    __syncwarp();
+    return f;
 }
 
-// Forms the treelet rooted at internal node r (one lane).
-__device__ void treelet_form(const float* __restrict__ nodes, const float4* __restrict__ leaf_boxes,
-                             const uint2* __restrict__ info, uint32_t n, uint32_t r, TreeletForm& f,
-                             uint32_t* __restrict__ status)
+__device__ __forceinline__ float treelet_cost(uint32_t address)
 {
-    f.internal_mask = 0;
-    f.inode[0] = r;
-    bool ok = treelet_take_children(nodes, leaf_boxes, info, n, r, 0, 1, f);
-    uint32_t m = 2, ni = 1;
-    float old = 0.f;
-    if (ok) {
-        float rb[6];
-        for (int a = 0; a < 3; ++a) {
-            rb[a] = fminf(f.box[0][a], f.box[1][a]);
-            rb[3 + a] = fmaxf(f.box[0][3 + a], f.box[1][3 + a]);
-        }
-        old = half_area(rb);
-    }
-    while (ok && m < (uint32_t)kTreeletLeaves) {
-        int b = -1;
-        float ba = -1.f;
-        for (uint32_t k = 0; k < m; ++k)
-            if ((f.internal_mask >> k) & 1u) {
-                const float a = half_area(f.box[k]);
-                if (a > ba) { ba = a; b = (int)k; }
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(address));
+    return v;
+}
+
+// Subsets of kK leaves listed at subs, each shared by kG lanes (at most 32 lanes in all): the
+// least c(P) + c(S \ P) over the splits P (with S's lowest leaf, P != S), the smallest P on
+// equal sums. A lane goes through its splits in ascending order (sub - rest & rest steps
+// through the subsets of rest); of kG lanes each fixes rest's highest log2(kG) leaves. Masks
+// are byte offsets into c (4 x the subset), or-ed onto its address.
+template <int kK, int kG>
+__device__ __forceinline__ void treelet_class(const uint8_t* subs, int count, uint32_t full, uint32_t c_at,
+                                              TreeletWarp& w)
+{
+    const int lane = threadIdx.x & 31;
+    const int rho = lane / kG;
+    const uint32_t S = rho < count ? subs[rho] : 0u;
+    const bool valid = S != 0u && !(S & ~full);
+    float best = INFINITY;
+    uint32_t bp = 0xFFFFFFFFu;
+    if (valid) {
+        const uint32_t low = S & (0u - S), S4 = 4u * S;
+        uint32_t rest = S ^ low, fixed = low;
+        if (kG > 1) {
+#pragma unroll
+            for (int g = kG / 2; g >= 1; g /= 2) {
+                const uint32_t top = 1u << (31 - __clz(rest));
+                rest ^= top;
+                if (lane & g) fixed |= top;
             }
-        if (b < 0) break;
-        f.inode[ni++] = f.id[b];
-        old = __fadd_rn(old, ba);
-        ok = treelet_take_children(nodes, leaf_boxes, info, n, f.id[b], b, (int)m, f);
-        ++m;
+        }
+        rest *= 4u;
+        fixed = c_at | 4u * fixed;
+        // kG == 1: every split but P == S, the last; else that one is the last lane's last, and
+        // (its lanes' first splits being real ones) is passed over by its sum
+        constexpr int kSteps = (1 << (kK - 1)) / kG - (kG == 1 ? 1 : 0);
+        uint32_t sub = 0;
+        if (kG == 1 || kSteps > 1 || fixed != (c_at | S4)) {
+            best = __fadd_rn(treelet_cost(fixed), treelet_cost(fixed ^ S4));
+            bp = fixed;
+        }
+#pragma unroll
+        for (int j = 1; j < kSteps; ++j) {
+            sub = (sub - rest) & rest;
+            const uint32_t P = fixed | sub;
+            float v = __fadd_rn(treelet_cost(P), treelet_cost(P ^ S4));
+            if (kG > 1 && j == kSteps - 1 && P == (c_at | S4)) v = INFINITY;
+            if (v < best) { best = v; bp = P; }
+        }
     }
-    if (!ok) atomicOr(status, CPT_STATUS_BAD_INDEX);
-    f.m = ok ? m : 0u;
-    f.old_cost = old;
+#pragma unroll
+    for (int o = 1; o < kG; o <<= 1) {
+        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+        const uint32_t op = __shfl_xor_sync(0xFFFFFFFFu, bp, o);
+        if (ov < best || (ov == best && op < bp)) { best = ov; bp = op; }
+    }
+    if (valid && (lane % kG) == 0) {
+        w.c[S] = __fadd_rn(w.c[S], best);
+        w.split[S] = (uint8_t)((bp >> 2) & 127u);
+    }
 }
 
 // Solves the warp's formed treelet (rooted at a node whose subtree is h_before tall)
 // and rewrites it if cheaper and no taller; called by the whole warp.
-__device__ void treelet_solve(float* __restrict__ nodes, uint32_t* __restrict__ parents_leaf,
-                              uint32_t* __restrict__ parents_internal, uint2* __restrict__ info,
-                              uint32_t h_before, const uint16_t* __restrict__ pairs, TreeletWarp& w)
+__device__ __forceinline__ void treelet_solve(float* __restrict__ nodes, uint32_t* __restrict__ parents_leaf,
+                                              uint32_t* __restrict__ parents_internal, uint2* __restrict__ info,
+                                              uint32_t h_before, const TreeletForm& f, const uint8_t* order,
+                                              TreeletWarp& w)
 {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();  // the form is written
-    const TreeletForm& f = w.form;
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t m = f.m;
-    if (m < 3) {
-        __syncwarp();  // every lane has read m before the next form is written
-        return;
-    }
+    if (m < 3) return;
     const uint32_t full = (1u << m) - 1u;
-    if ((uint32_t)lane < m) {
-        const uint32_t from = f.from[lane];
-        const float2* sp = reinterpret_cast<const float2*>(nodes + 24 * (size_t)(from >> 1) + 10 * (from & 1u));
-        for (int j = 0; j < 5; ++j) {
-            const float2 v = __ldcg(sp + j);
-            w.slot[lane][2 * j] = v.x;
-            w.slot[lane][2 * j + 1] = v.y;
-        }
-    }
-    for (uint32_t S = (uint32_t)lane + 1u; S <= full; S += 32u) {
-        if (__popc(S) == 1) { w.c[S] = 0.f; continue; }
+    // areas: the lane's bits pick among leaves 0-4, leaves 5 and 6 are added in turn
+    {
         float b[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+        auto add = [&](float (&x)[6], int k) {
 #pragma unroll
-        for (int k = 0; k < kTreeletLeaves; ++k)
-            if ((S >> k) & 1u)
+            for (int a = 0; a < 3; ++a) {
+                x[a] = fminf(x[a], w.box[k][a]);
+                x[3 + a] = fmaxf(x[3 + a], w.box[k][3 + a]);
+            }
+        };
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    b[a] = fminf(b[a], f.box[k][a]);
-                    b[3 + a] = fmaxf(b[3 + a], f.box[k][3 + a]);
-                }
-        w.c[S] = half_area(b);
+        for (int k = 0; k < 5; ++k)
+            if ((lane >> k) & 1u)
+                if (k < 3 || (uint32_t)k < m) add(b, k);
+        auto put = [&](const float (&x)[6], uint32_t S) {
+            if (S && !(S & ~full)) w.c[S] = __popc(S) == 1 ? 0.f : half_area(x);
+        };
+        put(b, lane);
+        if (m > 6) {
+            float c[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) c[a] = b[a];
+            add(c, 6);
+            put(c, lane | 64u);
+            add(c, 5);
+            put(c, lane | 96u);
+        }
+        if (m > 5) {
+            add(b, 5);
+            put(b, lane | 32u);
+        }
     }
     __syncwarp();
-    // size class k: C(7, k) subsets of 2^(k-1) - 1 splits each; a lane takes a subset,
-    // or (k = 6, 7) a group of g lanes shares a subset's splits and reduces by shuffles.
-    // The least (cost bits, split mask) wins.
-    for (int k = 2; k <= (int)m; ++k) {
-        const int subsets = k == 2 ? 21 : k == 3 ? 35 : k == 4 ? 35 : k == 5 ? 21 : k == 6 ? 7 : 1;
-        const int g = k == 6 ? 4 : k == 7 ? 32 : 1;
-        const int np = (1 << (k - 1)) - 1;
-        const uint16_t* cls = pairs + treelet_class_start(k);
-        for (int i0 = 0; i0 < subsets * g; i0 += 32) {
-            const int idx = i0 + lane, rho = idx / g, q = idx % g;
-            unsigned long long key = ~0ull;
-            uint32_t S = 0;
-            if (rho < subsets) {
-                const uint16_t* ps = cls + rho * np;
-                S = ps[0] & 127u;
-                if (!(S & ~full))
-                    for (int j = q; j < np; j += g) {
-                        const uint32_t P = (uint32_t)ps[j] >> 7;
-                        const float v = __fadd_rn(w.c[P], w.c[S ^ P]);
-                        const unsigned long long kk = ((unsigned long long)__float_as_uint(v) << 32) | P;
-                        key = kk < key ? kk : key;
-                    }
-            }
-            for (int o = 1; o < g; o <<= 1) {
-                const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, key, o);
-                key = other < key ? other : key;
-            }
-            if (rho < subsets && q == 0 && !(S & ~full)) {
-                w.c[S] = __fadd_rn(w.c[S], __uint_as_float((uint32_t)(key >> 32)));
-                w.split[S] = (uint8_t)(key & 127u);
-            }
-        }
+    // (the 33rd to 35th subsets of 3 and 4 leaves share lanes: 1 step instead of 3 and 7)
+    const uint32_t c_at = (uint32_t)__cvta_generic_to_shared(w.c);
+    treelet_class<2, 1>(order, 21, full, c_at, w);
+    __syncwarp();
+    treelet_class<3, 1>(order + 21, 32, full, c_at, w);
+    if (m > 6) treelet_class<3, 4>(order + 53, 3, full, c_at, w);
+    __syncwarp();
+    if (m > 3) {
+        treelet_class<4, 1>(order + 56, 32, full, c_at, w);
+        if (m > 6) treelet_class<4, 8>(order + 88, 3, full, c_at, w);
         __syncwarp();
     }
-    if (lane == 0 && w.c[full] < __fmul_rn(f.old_cost, 0.999999f)) {
-        // the new topology, top-down: node j covers subset sub[j]; a child reference
-        // is a treelet leaf k (< 8) or node 8 + j
-        uint32_t sub[kTreeletLeaves - 1], ck[kTreeletLeaves - 1][2];
+    if (m > 4) {
+        treelet_class<5, 1>(order + 91, 21, full, c_at, w);
+        __syncwarp();
+    }
+    if (m > 5) {
+        treelet_class<6, 4>(order + 112, 7, full, c_at, w);
+        __syncwarp();
+    }
+    if (m > 6) {
+        treelet_class<7, 32>(order + 119, 1, full, c_at, w);
+        __syncwarp();
+    }
+    if (!(w.c[full] < __fmul_rn(f.old_cost, 0.999999f))) return;
+    // the new topology, top-down
+    if (lane == 0) {
         uint32_t cnt = 1;
-        sub[0] = full;
-        bool ok = true;
-        for (uint32_t j = 0; j < cnt && ok; ++j) {
-            const uint32_t S = sub[j], P = w.split[S];
-            const uint32_t X[2] = {P, S ^ P};
+        w.sub[0] = (uint8_t)full;
+        w.node_depth[0] = 0;
+        for (uint32_t j = 0; j < cnt; ++j) {
+            const uint32_t S = w.sub[j], P = w.split[S], depth = w.node_depth[j] + 1u;
+#pragma unroll
             for (int side = 0; side < 2; ++side) {
-                if (X[side] == 0u || (X[side] & ~S)) { ok = false; break; }
-                if (__popc(X[side]) == 1) {
-                    ck[j][side] = (uint32_t)(__ffs(X[side]) - 1);
+                const uint32_t X = side ? S ^ P : P;
+                if (__popc(X) == 1) {
+                    const uint32_t k = (uint32_t)__ffs(X) - 1u;
+                    w.child[j][side] = (uint8_t)k;
+                    w.leaf_depth[k] = (uint8_t)depth;
                 } else {
-                    if (cnt >= m - 1) { ok = false; break; }
-                    sub[cnt] = X[side];
-                    ck[j][side] = 8u + cnt;
-                    ++cnt;
+                    w.child[j][side] = (uint8_t)(8u + cnt);
+                    w.sub[cnt] = (uint8_t)X;
+                    w.node_depth[cnt] = (uint8_t)depth;
+                    ++cnt;  // (a binary tree over m leaves has m - 1 nodes)
                 }
             }
         }
-        if (ok && cnt == m - 1) {
-            uint32_t h[kTreeletLeaves - 1], sz[kTreeletLeaves - 1];
-            for (int j = (int)cnt - 1; j >= 0; --j) {
-                uint32_t hh = 0, ss = 0;
-                for (int side = 0; side < 2; ++side) {
-                    const uint32_t c = ck[j][side];
-                    hh = max(hh, c < 8u ? f.height[c] : h[c - 8u]);
-                    ss += c < 8u ? f.size[c] : sz[c - 8u];
-                }
-                h[j] = hh + 1u;
-                sz[j] = ss;
-            }
-            if (h[0] <= h_before) {
-                for (uint32_t j = 0; j < cnt; ++j) {
-                    const uint32_t nd = f.inode[j];
-                    float* rec = nodes + 24 * (size_t)nd;
-                    uint32_t ids[2], word = 0;
-                    for (int side = 0; side < 2; ++side) {
-                        const uint32_t c = ck[j][side];
-                        float slot[10];
-                        if (c < 8u) {
-                            ids[side] = f.id[c];
-                            for (int a = 0; a < 10; ++a) slot[a] = w.slot[c][a];
-                            if ((f.internal_mask >> c) & 1u) {
-                                word |= 1u << side;
-                                parents_internal[ids[side]] = nd;
-                            } else {
-                                parents_leaf[ids[side]] = nd;
-                            }
-                        } else {
-                            const uint32_t x = c - 8u, X = sub[x];
-                            ids[side] = f.inode[x];
-                            word |= 1u << side;
-                            for (int a = 0; a < 3; ++a) { slot[a] = FLT_MAX; slot[3 + a] = -FLT_MAX; }
-                            for (uint32_t k = 0; k < m; ++k)
-                                if ((X >> k) & 1u)
-                                    for (int a = 0; a < 3; ++a) {
-                                        slot[a] = fminf(slot[a], f.box[k][a]);
-                                        slot[3 + a] = fmaxf(slot[3 + a], f.box[k][3 + a]);
-                                    }
-                            slot[6] = slot[7] = slot[8] = slot[9] = 0.0f;
-                            parents_internal[ids[side]] = nd;
-                        }
-                        store_slot(rec, side, slot);
-                    }
-                    word |= ids[0] << 2;
-                    reinterpret_cast<float4*>(rec)[5] =
-                        make_float4(__uint_as_float(word), __uint_as_float(ids[1]), 0.f, 0.f);
-                    info[nd] = make_uint2(sz[j], h[j]);
-                }
-            }
-        }
-        __threadfence();
     }
     __syncwarp();
+    // lanes 2 j and 2 j + 1: the two children of node j
+    const uint32_t j = lane >> 1, side = lane & 1u;
+    const bool mine = j < m - 1u;
+    uint32_t h = 0, sz = 0;
+    if (mine) {
+        const uint32_t S = w.sub[j], d = w.node_depth[j];
+        for (uint32_t k = 0; k < m; ++k)
+            if ((S >> k) & 1u) {
+                h = max(h, w.height[k] + w.leaf_depth[k] - d);
+                sz += w.size[k];
+            }
+    }
+    if (__shfl_sync(0xFFFFFFFFu, h, 0) > h_before) return;
+    const uint32_t nd = mine ? w.inode[j] : 0u;
+    uint32_t id = 0, bit = 0;
+    if (mine) {
+        const uint32_t c = w.child[j][side];
+        float2* out = reinterpret_cast<float2*>(nodes + 24 * (size_t)nd + 10 * side);
+        if (c < 8u) {
+            id = w.id[c];
+            const float2* s2 = reinterpret_cast<const float2*>(w.slot[c]);
+#pragma unroll
+            for (int a = 0; a < 5; ++a) out[a] = s2[a];
+            bit = (f.internal_mask >> c) & 1u;
+            (bit ? parents_internal : parents_leaf)[id] = nd;
+        } else {
+            const uint32_t X = w.sub[c - 8u];
+            id = w.inode[c - 8u];
+            bit = 1u;
+            float b[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+            for (uint32_t k = 0; k < m; ++k)
+                if ((X >> k) & 1u)
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        b[a] = fminf(b[a], w.box[k][a]);
+                        b[3 + a] = fmaxf(b[3 + a], w.box[k][3 + a]);
+                    }
+            out[0] = make_float2(b[0], b[1]);
+            out[1] = make_float2(b[2], b[3]);
+            out[2] = make_float2(b[4], b[5]);
+            out[3] = out[4] = make_float2(0.f, 0.f);
+            parents_internal[id] = nd;
+        }
+    }
+    const uint32_t rid = __shfl_xor_sync(0xFFFFFFFFu, id, 1), rbit = __shfl_xor_sync(0xFFFFFFFFu, bit, 1);
+    if (mine && side == 0u) {
+        const uint32_t word = (id << 2) | (rbit << 1) | bit;
+        reinterpret_cast<float4*>(nodes + 24 * (size_t)nd)[5] =
+            make_float4(__uint_as_float(word), __uint_as_float(rid), 0.f, 0.f);
+        info[nd] = make_uint2(sz, h);
+    }
+    __threadfence();
+    __syncwarp();  // the climbing lane's arrival at the next node releases every lane's stores
 }
 
 // A round of treelet restructuring over the split tree: every piece's walker goes
 // up; the second arrival at a node records its size and height and, at gamma or
 // more leaves, has its warp form and solve the node's treelet.
-__global__ void __launch_bounds__(kTreeletBlock) k_treelet(const uint32_t* __restrict__ n_pieces,
+//
+// Issue-bound (67 % of cycles) and behind it the chain of a treelet's dependent fetches. The
+// whole warp forms, solves and rewrites a treelet: 11.8 M pieces (1.3 M-triangle hairball
+// scene, ratio 8.0) in 12.0 ms against 23.8 when lane 0 gathered the leaves and wrote the
+// new topology alone and the splits came from a table; the trees are the same bytes. 10
+// blocks per SM (48 registers): with 9 the scene's whole build took 24.8 ms, with 10 24.6,
+// with 12 25.1, with 16 (32 registers, spills) 26.4.
+__global__ void __launch_bounds__(kTreeletBlock, 10) k_treelet(const uint32_t* __restrict__ n_pieces,
                                                           float* __restrict__ nodes,
                                                           const float4* __restrict__ leaf_boxes,
                                                           uint32_t* __restrict__ parents_leaf,
@@ -800,36 +869,13 @@ __global__ void __launch_bounds__(kTreeletBlock) k_treelet(const uint32_t* __res
                                                           int* __restrict__ counters, uint2* __restrict__ info,
                                                           uint32_t gamma, uint32_t* __restrict__ status)
 {
-    // (subset, split) pairs by subset size: a subset S of k >= 2 leaves lists its
-    // 2^(k-1) - 1 splits P (P holds S's lowest leaf, P != S) from
-    // treelet_class_start(k) + rank of S among the k-leaf subsets x (2^(k-1) - 1).
-    __shared__ uint16_t s_pairs[kTreeletPairs];
+    __shared__ uint8_t s_order[120];
     __shared__ TreeletWarp s_warp[kTreeletWarps];
-    if (threadIdx.x < kTreeletSubsets) {
-        const uint32_t S = threadIdx.x;
-        const int k = __popc(S);
-        if (k >= 2) {
-            uint32_t rank = 0;
-            for (uint32_t x = 1; x < S; ++x) rank += __popc(x) == k ? 1u : 0u;
-            const uint32_t np = (1u << (k - 1)) - 1u, low = S & (0u - S), rest = S ^ low;
-            uint16_t* out = s_pairs + treelet_class_start(k) + rank * np;
-            for (uint32_t j = 0; j < np; ++j) {
-                uint32_t P = low, bits = rest, jj = j;
-                while (bits) {
-                    const uint32_t b = bits & (0u - bits);
-                    if (jj & 1u) P |= b;
-                    jj >>= 1;
-                    bits ^= b;
-                }
-                out[j] = (uint16_t)(S | (P << 7));
-            }
-        }
-    }
+    if (threadIdx.x < 120) s_order[threadIdx.x] = kTreeletOrder[threadIdx.x];
     __syncthreads();
     const uint32_t n = *n_pieces;
     if (n < 3) return;
     if (sort_timed_out(status)) return;  // (uniform over the launch: set before it started)
-    const int lane = threadIdx.x & 31;
     TreeletWarp& w = s_warp[threadIdx.x >> 5];
     const uint32_t i = blockIdx.x * kTreeletBlock + threadIdx.x;
     bool active = i < n;
@@ -883,8 +929,8 @@ __global__ void __launch_bounds__(kTreeletBlock) k_treelet(const uint32_t* __res
             todo &= todo - 1u;
             const uint32_t r = __shfl_sync(0xFFFFFFFFu, node, src);
             const uint32_t hr = __shfl_sync(0xFFFFFFFFu, height, src);
-            if (lane == 0) treelet_form(nodes, leaf_boxes, info, n, r, w.form, status);
-            treelet_solve(nodes, parents_leaf, parents_internal, info, hr, s_pairs, w);
+            const TreeletForm f = treelet_form(nodes, leaf_boxes, info, n, r, w, status);
+            treelet_solve(nodes, parents_leaf, parents_internal, info, hr, f, s_order, w);
         }
         if (active) node = __ldcg(parents_internal + node);
     }
