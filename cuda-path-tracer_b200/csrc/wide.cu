@@ -115,18 +115,15 @@ __device__ __forceinline__ float box_area(const float* b)
     return dx * dy + dy * dz + dz * dx;
 }
 
-// Child `side` of the binary node whose record is w and whose box is pb: its box and
-// reference (internal: its binary index; leaf: parent * 2 + side | kLeafRef).
-__device__ __forceinline__ void child_of(const float w[24], uint32_t parent, const float pb[6], int side, float box[6],
-                                         uint32_t& ref)
+// A child of binary node `parent` (box pb) from its slot words s: its box and reference
+// (internal: its binary index; leaf: parent * 2 + side | kLeafRef).
+__device__ __forceinline__ void child_of_slot(const float s[10], bool internal, uint32_t index, uint32_t parent,
+                                              const float pb[6], int side, float box[6], uint32_t& ref)
 {
-    const uint32_t word = __float_as_uint(w[20]);
-    const bool internal = side ? (word & 2u) : (word & 1u);
-    const float* s = w + 10 * side;
     if (internal) {
 #pragma unroll
         for (int k = 0; k < 6; ++k) box[k] = s[k];
-        ref = side ? __float_as_uint(w[21]) : (word >> 2);
+        ref = index;
     } else {
         const float v0[3] = {s[0], s[1], s[2]};
 #pragma unroll
@@ -138,6 +135,15 @@ __device__ __forceinline__ void child_of(const float w[24], uint32_t parent, con
         }
         ref = (2u * parent + (uint32_t)side) | kLeafRef;
     }
+}
+
+// Child `side` of the binary node whose record is w.
+__device__ __forceinline__ void child_of(const float w[24], uint32_t parent, const float pb[6], int side, float box[6],
+                                         uint32_t& ref)
+{
+    const uint32_t word = __float_as_uint(w[20]);
+    child_of_slot(w + 10 * side, side ? (word & 2u) : (word & 1u), side ? __float_as_uint(w[21]) : (word >> 2), parent,
+                  pb, side, box, ref);
 }
 
 // The root of the wide tree queued (level 0), the counters zeroed, the margin m.
@@ -321,7 +327,10 @@ __device__ void sah_node(const float4* __restrict__ bin, uint32_t bin_internal, 
 }
 
 // The cost tables bottom-up: a walk starts at every node with two leaf children and goes
-// up while it is the last of a node's internal children to arrive (as the refit).
+// up while it is the last of a node's internal children to arrive (as the refit). Bound by
+// the latency of a step's dependent fetches and its release, so by the walks in flight: eight
+// lanes to a walk (a cost each, 4 walks a warp) ran 40 % slower; one acquire-release
+// arrival in place of two fences took 11.8 M nodes from 2.15 to 1.85 ms.
 __global__ void k_sah_up(const float4* __restrict__ bin, uint32_t bin_internal, const uint32_t* __restrict__ parent,
                          uint32_t* __restrict__ arrive, uint32_t* __restrict__ choice, float* __restrict__ cost,
                          uint32_t* __restrict__ status)
@@ -334,10 +343,8 @@ __global__ void k_sah_up(const float4* __restrict__ bin, uint32_t bin_internal, 
         sah_node(bin, bin_internal, parent, choice, cost, n);
         const uint32_t p = parent[n];
         if (p >= bin_internal) return;  // the root
-        __threadfence();
         const uint32_t need = __popc(__float_as_uint(bin[6 * (size_t)p + 5].x) & 3u);
-        if (atomicAdd(&arrive[p], 1u) + 1u < need) return;
-        __threadfence();
+        if ((uint32_t)arrive_acq_rel(reinterpret_cast<int*>(arrive + p)) + 1u < need) return;
         n = p;
     }
     atomicOr(status, CPT_STATUS_BAD_INDEX);  // a cycle: not a tree
@@ -355,209 +362,269 @@ __device__ __forceinline__ int scale_exp(double ext)
     return max(-126, min(127, e));
 }
 
-// The wide nodes [start, end) of one level: each collapses its binary subtree into up
-// to 8 children, allocates its internal children (queued as the next level) and its
-// leaf records.
+constexpr uint32_t kAll = 0xFFFFFFFFu;
+constexpr int kWideGroups = kWideBlock / 8;
+struct WideStage {  // a block's node planes: per group and axis, slot s's (lo, hi) bytes at halfword s
+    uint32_t planes[kWideGroups][3][4];
+};
+
+// Child `side` of the binary node at record index c whose box is pb, loaded by one lane.
+__device__ __forceinline__ void load_child(const float4* __restrict__ bin, uint32_t c, const float pb[6], int side,
+                                           float box[6], uint32_t& ref)
+{
+    const float4 meta = bin[6 * (size_t)c + 5];
+    const float2* s2 = reinterpret_cast<const float2*>(bin + 6 * (size_t)c) + 5 * side;
+    float w[10];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const float2 v = s2[k];
+        w[2 * k] = v.x;
+        w[2 * k + 1] = v.y;
+    }
+    const uint32_t word = __float_as_uint(meta.x);
+    child_of_slot(w, side ? (word & 2u) : (word & 1u), side ? __float_as_uint(meta.y) : (word >> 2), c, pb, side, box,
+                  ref);
+}
+
+// The wide nodes [start, end) of one level, eight lanes per node: lane i of a group holds the
+// node's child i (box, binary reference) while the collapse opens up to 8 of them, then
+// quantizes it, writes its triangle records or queues it for the next level. The groups of
+// a warp go through the steps together.
+//
+// What bounded the form with a thread per node was its serial work (7 of 32 lanes active, 14 %
+// of issue slots used: eight dependent record fetches, 8 x 8 x 8 slot costs and 48 double
+// quantizations one after the other) and one atomic per node and counter on the same two
+// words; here a warp's four nodes take one. 1.7 M wide nodes over 11.8 M leaves: 5.07 -> 1.60
+// ms; twelve small trees in one batch: 1,026 -> 410 us; the same nodes and records.
 __device__ __forceinline__ void wide_level_nodes(const float4* __restrict__ bin, float4* __restrict__ wide,
                                                  float4* __restrict__ tris, float4* __restrict__ queue,
                                                  uint32_t* __restrict__ ctr, uint32_t start, uint32_t end, float m,
                                                  uint32_t node_cap, uint32_t tri_cap, uint32_t bin_internal,
-                                                 uint32_t* __restrict__ status, float (*s_box)[kWideBlock],
-                                                 uint32_t (*s_ref)[kWideBlock],
+                                                 uint32_t* __restrict__ status, WideStage& stage,
                                                  const uint32_t* __restrict__ choice,  // null: the greedy collapse
-                                                 uint32_t rot = 0)  // node start + j goes to thread (j + rot) mod T
+                                                 uint32_t rot = 0)  // node start + j goes to group (j + rot) mod G
 {
-    const int t = threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, i = lane & 7u;
+    uint32_t (&planes)[3][4] = stage.planes[threadIdx.x >> 3];
     if (end > node_cap) {  // (only when the binary tree was not one: allocations past the cap were refused)
-        if (blockIdx.x == 0 && t == 0) atomicOr(status, CPT_STATUS_BAD_INDEX);
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, CPT_STATUS_BAD_INDEX);
         end = node_cap;
     }
-    const uint32_t nt = gridDim.x * kWideBlock, tid = blockIdx.x * kWideBlock + t;
-    const uint32_t first = (tid + nt - rot % nt) % nt;
-    for (uint32_t wi = start + first; wi < end; wi += nt) {
-        const float4 q0 = queue[2 * (size_t)wi], q1 = queue[2 * (size_t)wi + 1];
-        const uint32_t b = __float_as_uint(q0.w);
-        const float nb[6] = {q0.x, q0.y, q0.z, q1.x, q1.y, q1.z};
-        if (b >= bin_internal) { atomicOr(status, CPT_STATUS_BAD_INDEX); continue; }
-        int count = 0;
-        if (choice) {
-            // frontier: the binary node's children with the budgets of D(b, 8), then every
-            // child whose budget (after the C(n, j) = C(n, j - 1) steps) is 2 or more is
-            // replaced by its own two children with the budgets of its D(n, j)
-            int budget[8];
-            {
-                float w[24];
-                read_record(bin, b, w);
-                const int k = sah_split(__ldcg(choice + b), 8);
-                for (int side = 0; side < 2; ++side) {
-                    float bx[6];
-                    uint32_t ref;
-                    child_of(w, b, nb, side, bx, ref);
-                    for (int q = 0; q < 6; ++q) s_box[6 * count + q][t] = bx[q];
-                    s_ref[count][t] = ref;
-                    budget[count] = side ? 8 - k : k;
-                    ++count;
-                }
+    const uint32_t ng = gridDim.x * kWideGroups, gid = blockIdx.x * kWideGroups + (threadIdx.x >> 3);
+    const uint32_t first = (gid + ng - rot % ng) % ng;
+    for (uint32_t j = first;; j += ng) {
+        bool on = start < end && j < end - start;  // (the same in all lanes of a group)
+        if (!__any_sync(kAll, on)) break;
+        const uint32_t wi = start + j;
+        float nb[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        uint32_t b = 0;
+        if (on) {
+            const float4 q0 = queue[2 * (size_t)wi], q1 = queue[2 * (size_t)wi + 1];
+            b = __float_as_uint(q0.w);
+            nb[0] = q0.x; nb[1] = q0.y; nb[2] = q0.z; nb[3] = q1.x; nb[4] = q1.y; nb[5] = q1.z;
+            if (b >= bin_internal) {
+                if (i == 0) atomicOr(status, CPT_STATUS_BAD_INDEX);
+                on = false;
             }
-            for (int i = 0; i < count;) {
-                const uint32_t c = s_ref[i][t];
-                if ((c & kLeafRef) || c >= bin_internal) { ++i; continue; }
-                const uint32_t cc = __ldcg(choice + c);
-                int j = budget[i];
-                while (j >= 2 && sah_reduce(cc, j)) --j;
-                if (j < 2 || count >= 8) { ++i; continue; }  // one child: a wide node or a leaf slot
-                const int k = sah_split(cc, j);
-                float pb[6];
-                for (int q = 0; q < 6; ++q) pb[q] = s_box[6 * i + q][t];
-                float w[24];
-                read_record(bin, c, w);
-                for (int side = 0; side < 2; ++side) {
-                    float bx[6];
-                    uint32_t ref;
-                    child_of(w, c, pb, side, bx, ref);
-                    const int slot = side == 0 ? i : count++;
-                    for (int q = 0; q < 6; ++q) s_box[6 * slot + q][t] = bx[q];
-                    s_ref[slot][t] = ref;
-                    budget[slot] = side ? j - k : k;
+        }
+        float box[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        uint32_t ref = kLeafRef, cc = 0, budget = 0;
+        uint32_t count = on ? 2u : 0u;
+        if (on && i < 2u) load_child(bin, b, nb, (int)i, box, ref);
+        if (choice && on) {
+            const int k = sah_split(__ldcg(choice + b), 8);
+            budget = i == 0 ? k : 8 - k;
+            if (i < 2u && !(ref & kLeafRef) && ref < bin_internal) cc = __ldcg(choice + ref);
+        }
+        // open children: with costs, every child whose budget (after the C(n, j) = C(n, j - 1)
+        // steps) is 2 or more, in turn, gives way to its own two with the budgets of its
+        // D(n, j); else the internal child of largest area until there are 8
+        uint32_t at = 0;
+        for (bool more = on; __any_sync(kAll, more);) {
+            uint32_t open = 0;
+            int jb = 0;
+            if (choice) {
+                // the lane's own budget after the C(n, j) = C(n, j - 1) steps; below 2: one child
+                jb = (int)budget;
+                const bool splits = i < count && !(ref & kLeafRef) && ref < bin_internal;
+                if (splits)
+                    while (jb >= 2 && sah_reduce(cc, jb)) --jb;
+                const uint32_t want = __ballot_sync(kAll, splits && jb >= 2 && i >= at) >> (lane & 24u) & 0xFFu;
+                more = more && want != 0u && count < 8u;
+                open = want ? (uint32_t)__ffs(want) - 1u : 0u;
+                if (more) at = open;
+            } else {
+                float a = -1.f;
+                if (i < count && !(ref & kLeafRef)) {
+                    const float x = box_area(box);
+                    a = x > -1.f ? x : -1.f;
                 }
+                uint32_t who = i;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const float oa = __shfl_xor_sync(kAll, a, o);
+                    const uint32_t ow = __shfl_xor_sync(kAll, who, o);
+                    if (oa > a || (oa == a && ow < who)) { a = oa; who = ow; }
+                }
+                more = more && a > -1.f && count < 8u;
+                open = who;
             }
-        } else {
-            // frontier: the binary node's children, then open the largest internal one
-            {
-                float w[24];
-                read_record(bin, b, w);
-                for (int side = 0; side < 2; ++side) {
-                    float bx[6];
-                    uint32_t ref;
-                    child_of(w, b, nb, side, bx, ref);
-                    for (int k = 0; k < 6; ++k) s_box[6 * count + k][t] = bx[k];
-                    s_ref[count][t] = ref;
-                    ++count;
-                }
+            const uint32_t c = __shfl_sync(kAll, ref, open, 8);
+            const int jo = __shfl_sync(kAll, jb, open, 8);
+            const uint32_t co = __shfl_sync(kAll, cc, open, 8);
+            float pb[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) pb[k] = __shfl_sync(kAll, box[k], open, 8);
+            if (more && c >= bin_internal) {  // (greedy only: the costs' collapse passed it over)
+                if (i == 0) atomicOr(status, CPT_STATUS_BAD_INDEX);
+                more = false;
             }
-            while (count < 8) {
-                int best = -1;
-                float best_area = -1.f;
-                for (int i = 0; i < count; ++i) {
-                    if (s_ref[i][t] & kLeafRef) continue;
-                    float bx[6];
-                    for (int k = 0; k < 6; ++k) bx[k] = s_box[6 * i + k][t];
-                    const float a = box_area(bx);
-                    if (a > best_area) { best_area = a; best = i; }
-                }
-                if (best < 0) break;
-                const uint32_t c = s_ref[best][t];
-                if (c >= bin_internal) { atomicOr(status, CPT_STATUS_BAD_INDEX); break; }
-                float pb[6];
-                for (int k = 0; k < 6; ++k) pb[k] = s_box[6 * best + k][t];
-                float w[24];
-                read_record(bin, c, w);
-                for (int side = 0; side < 2; ++side) {
-                    float bx[6];
-                    uint32_t ref;
-                    child_of(w, c, pb, side, bx, ref);
-                    const int slot = side == 0 ? best : count++;
-                    for (int k = 0; k < 6; ++k) s_box[6 * slot + k][t] = bx[k];
-                    s_ref[slot][t] = ref;
+            if (more) {
+                const uint32_t added = count++;
+                if (i == open || i == added) {
+                    load_child(bin, c, pb, i == added ? 1 : 0, box, ref);
+                    if (choice) {
+                        const int k = sah_split(co, jo);
+                        budget = i == added ? jo - k : k;
+                        cc = !(ref & kLeafRef) && ref < bin_internal ? __ldcg(choice + ref) : 0u;
+                    }
                 }
             }
         }
-        // quantization frame
+        // quantization frame: lane a < 3 has axis a
+        float pf = 0.f;
+        int ea = 0;
+        if (i < 3u) {
+            const float l = i == 0 ? nb[0] : i == 1 ? nb[1] : nb[2], h = i == 0 ? nb[3] : i == 1 ? nb[4] : nb[5];
+            const double lo = (double)l - (double)m, hi = (double)h + (double)m;
+            ea = scale_exp((hi - lo) * (1.0 + 1e-6));
+            // p one quantum below the widened box, rounded down to a float
+            const double pd = lo - ldexp(1.0, ea);
+            pf = (float)pd;
+            if ((double)pf > pd) pf = nextafterf(pf, -FLT_MAX);
+        }
         float p[3];
         int e[3];
-        double sc[3];
-        float ctr_b[3];
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const double lo = (double)nb[a] - (double)m, hi = (double)nb[3 + a] + (double)m;
-            e[a] = scale_exp((hi - lo) * (1.0 + 1e-6));
-            sc[a] = ldexp(1.0, e[a]);
-            // p one quantum below the widened box, rounded down to a float
-            const double pd = lo - sc[a];
-            float pf = (float)pd;
-            if ((double)pf > pd) pf = nextafterf(pf, -FLT_MAX);
-            p[a] = pf;
-            ctr_b[a] = 0.5f * (nb[a] + nb[3 + a]);
+            p[a] = __shfl_sync(kAll, pf, a, 8);
+            e[a] = __shfl_sync(kAll, ea, a, 8);
         }
-        // slots by direction: greedy smallest projection on the octant diagonal
-        int slot_of[8];
-        uint32_t used = 0, placed = 0;
-        for (int i = 0; i < count; ++i) slot_of[i] = -1;
-        for (int r = 0; r < count; ++r) {
-            float best_c = FLT_MAX;
-            int bi = 0, bs = 0;
-            for (int i = 0; i < count; ++i) {
-                if (placed >> i & 1u) continue;
-                float c[3];
-                for (int a = 0; a < 3; ++a) c[a] = 0.5f * (s_box[6 * i + a][t] + s_box[6 * i + 3 + a][t]) - ctr_b[a];
-                for (int s = 0; s < 8; ++s) {
-                    if (used >> s & 1u) continue;
-                    const float cost = ((s & 1) ? -c[0] : c[0]) + ((s & 2) ? -c[1] : c[1]) + ((s & 4) ? -c[2] : c[2]);
-                    if (cost < best_c) { best_c = cost; bi = i; bs = s; }
+        // slots by direction: greedily the smallest projection on an octant's diagonal, the
+        // first child and the first slot of equal ones
+        const bool child = i < count;
+        uint32_t slot = 8u, used = 0;
+        {
+            float cst[8];
+            float cen[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) cen[a] = 0.5f * (box[a] + box[3 + a]) - 0.5f * (nb[a] + nb[3 + a]);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                cst[q] = ((q & 1) ? -cen[0] : cen[0]) + ((q & 2) ? -cen[1] : cen[1]) + ((q & 4) ? -cen[2] : cen[2]);
+            const uint32_t rounds = __reduce_max_sync(kAll, count);
+            for (uint32_t r = 0; r < rounds; ++r) {
+                float best = INFINITY;
+                uint32_t key = (i << 3) | 7u;
+                if (child && slot == 8u) {
+                    const uint32_t unused = ~used & 0xFFu;
+                    key = (i << 3) | ((uint32_t)__ffs(unused) - 1u);
+                    best = FLT_MAX;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (!((used >> q) & 1u) && cst[q] < best) { best = cst[q]; key = (i << 3) | (uint32_t)q; }
+                }
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const float ob = __shfl_xor_sync(kAll, best, o);
+                    const uint32_t ok = __shfl_xor_sync(kAll, key, o);
+                    if (ob < best || (ob == best && ok < key)) { best = ob; key = ok; }
+                }
+                if (r < count) {
+                    used |= 1u << (key & 7u);
+                    if ((key >> 3) == i) slot = key & 7u;
                 }
             }
-            slot_of[bi] = bs;
-            placed |= 1u << bi;
-            used |= 1u << bs;
         }
         // leaf slots (m1) and those holding a second (m2) and third (m3) record; the
         // node's records are layers of n_leaf records, one per leaf slot in slot order
-        uint32_t cnt_of[8];
-        uint32_t imask = 0, m1 = 0, m2 = 0, m3 = 0;
-        for (int i = 0; i < count; ++i) {
-            const uint32_t ref = s_ref[i][t];
-            cnt_of[i] = (!choice || (ref & kLeafRef) || (ref < bin_internal && sah_leaf(__ldcg(choice + ref))))
-                            ? leaf_records(bin, ref, bin_internal)
-                            : 0u;
-            const uint32_t bit = 1u << slot_of[i];
-            if (!cnt_of[i]) imask |= bit;
-            if (cnt_of[i] >= 1) m1 |= bit;
-            if (cnt_of[i] >= 2) m2 |= bit;
-            if (cnt_of[i] >= 3) m3 |= bit;
+        uint32_t cnt = 0;
+        if (child && (!choice || (ref & kLeafRef) || (ref < bin_internal && sah_leaf(cc))))
+            cnt = leaf_records(bin, ref, bin_internal);
+        uint32_t masks = 0;
+        if (child) {
+            const uint32_t bit = 1u << slot;
+            masks = cnt ? (bit << 8) | (cnt >= 2u ? bit << 16 : 0u) | (cnt >= 3u ? bit << 24 : 0u) : bit;
         }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) masks |= __shfl_xor_sync(kAll, masks, o);
+        const uint32_t imask = masks & 0xFFu, m1 = (masks >> 8) & 0xFFu, m2 = (masks >> 16) & 0xFFu, m3 = masks >> 24;
         const uint32_t n_int = __popc(imask), n_leaf = __popc(m1);
         const uint32_t n_rec = n_leaf * (m3 ? 3u : m2 ? 2u : 1u);
-        const uint32_t child_base = n_int ? atomicAdd(&ctr[0], n_int) : 0u;
-        const uint32_t tri_base = n_rec ? atomicAdd(&ctr[1], n_rec) : 0u;
-        if (child_base + n_int > node_cap || tri_base + n_rec > tri_cap) {
-            atomicOr(status, CPT_STATUS_BAD_INDEX);
-            continue;
+        // allocation: one 64-bit add per warp to (wide nodes, records)
+        uint32_t before_int = 0, before_rec = 0, all_int = 0, all_rec = 0;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const uint32_t gi = __shfl_sync(kAll, n_int, 8 * g), gr = __shfl_sync(kAll, n_rec, 8 * g);
+            if (8u * g < (lane & 24u)) { before_int += gi; before_rec += gr; }
+            all_int += gi;
+            all_rec += gr;
         }
-        // per axis, word j: slots 2j, 2j+1 as bytes (lo, hi, lo, hi); an empty slot is (255, 0)
-        uint32_t qp[3][4];
-        for (int a = 0; a < 3; ++a)
-            for (int j = 0; j < 4; ++j) qp[a][j] = 0x00FF00FFu;
-        for (int i = 0; i < count; ++i) {
-            const int s = slot_of[i];
-            const uint32_t ref = s_ref[i][t];
-            float bx[6];
-            for (int k = 0; k < 6; ++k) bx[k] = s_box[6 * i + k][t];
+        unsigned long long got = 0;
+        if (lane == 0 && (all_int | all_rec))
+            got = atomicAdd(reinterpret_cast<unsigned long long*>(ctr),
+                            (unsigned long long)all_int | ((unsigned long long)all_rec << 32));
+        got = __shfl_sync(kAll, got, 0);
+        const uint32_t child_base = n_int ? (uint32_t)got + before_int : 0u;
+        const uint32_t tri_base = n_rec ? (uint32_t)(got >> 32) + before_rec : 0u;
+        if (on && (child_base + n_int > node_cap || tri_base + n_rec > tri_cap)) {
+            if (i == 0) atomicOr(status, CPT_STATUS_BAD_INDEX);
+            on = false;
+        }
+        // planes: an empty slot is (255, 0)
+        if (i < 4u)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) planes[a][i] = 0x00FF00FFu;
+        __syncwarp();
+        if (child) {
+#pragma unroll
             for (int a = 0; a < 3; ++a) {
                 // one quantum of slack each side for the traversal's folded plane offset
-                const double lo = (double)bx[a] - (double)m, hi = (double)bx[3 + a] + (double)m;
-                const int ql = (int)fmin(fmax(floor((lo - (double)p[a]) / sc[a]) - 1.0, 0.0), 255.0);
-                const int qh = (int)fmin(fmax(ceil((hi - (double)p[a]) / sc[a]) + 1.0, 0.0), 255.0);
-                const int sh = 16 * (s & 1);
-                qp[a][s >> 1] = (qp[a][s >> 1] & ~(0xFFFFu << sh)) | (((uint32_t)ql | ((uint32_t)qh << 8)) << sh);
-            }
-            const uint32_t below = (1u << s) - 1u;
-            if (cnt_of[i]) {
-                emit_records(bin, ref, cnt_of[i], tris + 3 * (size_t)(tri_base + __popc(m1 & below)), n_leaf);
-            } else {
-                float4* qd = queue + 2 * (size_t)(child_base + __popc(imask & below));
-                qd[0] = make_float4(bx[0], bx[1], bx[2], __uint_as_float(ref));
-                qd[1] = make_float4(bx[3], bx[4], bx[5], 0.f);
+                const double inv = ldexp(1.0, -e[a]);  // (a division by 2^e, exact)
+                const double lo = (double)box[a] - (double)m, hi = (double)box[3 + a] + (double)m;
+                const int ql = (int)fmin(fmax(floor((lo - (double)p[a]) * inv) - 1.0, 0.0), 255.0);
+                const int qh = (int)fmin(fmax(ceil((hi - (double)p[a]) * inv) + 1.0, 0.0), 255.0);
+                reinterpret_cast<uint16_t*>(planes[a])[slot] = (uint16_t)((uint32_t)ql | ((uint32_t)qh << 8));
             }
         }
-        // the scale 2^e of an axis as the high half-word of its float bits: (e + 127) << 7
-        const uint32_t hx = (uint32_t)(e[0] + 127) << 7, hy = (uint32_t)(e[1] + 127) << 7,
-                       hz = (uint32_t)(e[2] + 127) << 7;
-        float4* o = wide + 5 * (size_t)wi;
-        o[0] = make_float4(p[0], p[1], p[2], __uint_as_float(hz | (imask << 24)));
-        o[1] = make_float4(__uint_as_float(child_base), __uint_as_float(tri_base),
-                           __uint_as_float(m1 | (m2 << 8) | (m3 << 16)), __uint_as_float(hx | (hy << 16)));
-        for (int a = 0; a < 3; ++a)
-            o[2 + a] = make_float4(__uint_as_float(qp[a][0]), __uint_as_float(qp[a][1]), __uint_as_float(qp[a][2]),
-                                   __uint_as_float(qp[a][3]));
+        __syncwarp();
+        if (on) {
+            if (child) {
+                const uint32_t below = (1u << slot) - 1u;
+                if (cnt) {
+                    emit_records(bin, ref, cnt, tris + 3 * (size_t)(tri_base + __popc(m1 & below)), n_leaf);
+                } else {
+                    float4* qd = queue + 2 * (size_t)(child_base + __popc(imask & below));
+                    qd[0] = make_float4(box[0], box[1], box[2], __uint_as_float(ref));
+                    qd[1] = make_float4(box[3], box[4], box[5], 0.f);
+                }
+            }
+            // the scale 2^e of an axis as the high half-word of its float bits: (e + 127) << 7
+            if (i < 5u) {
+                const uint32_t hx = (uint32_t)(e[0] + 127) << 7, hy = (uint32_t)(e[1] + 127) << 7,
+                               hz = (uint32_t)(e[2] + 127) << 7;
+                float4 v;
+                if (i == 0) v = make_float4(p[0], p[1], p[2], __uint_as_float(hz | (imask << 24)));
+                else if (i == 1)
+                    v = make_float4(__uint_as_float(child_base), __uint_as_float(tri_base),
+                                    __uint_as_float(m1 | (m2 << 8) | (m3 << 16)), __uint_as_float(hx | (hy << 16)));
+                else
+                    v = make_float4(__uint_as_float(planes[i - 2][0]), __uint_as_float(planes[i - 2][1]),
+                                    __uint_as_float(planes[i - 2][2]), __uint_as_float(planes[i - 2][3]));
+                wide[5 * (size_t)wi + i] = v;
+            }
+        }
+        __syncwarp();  // the planes are read
     }
 }
 
@@ -576,8 +643,7 @@ __global__ void __launch_bounds__(kWideBlock) k_wide_levels(const float4* __rest
                                                             uint32_t* __restrict__ status,
                                                             const uint32_t* __restrict__ choice)
 {
-    __shared__ float s_box[8 * 6][kWideBlock];
-    __shared__ uint32_t s_ref[8][kWideBlock];
+    __shared__ WideStage s_stage;
     // A sort of the build (or of the split tree) gave up a look-back wait: the binary
     // tree is not one. Every block leaves at once (the word was set before this launch,
     // so all see it and none waits at the barrier), and no node is written.
@@ -587,8 +653,8 @@ __global__ void __launch_bounds__(kWideBlock) k_wide_levels(const float4* __rest
     uint32_t start = 0, end = 1;  // level 0: the root, queued by k_wide_init
     int level = 0;
     for (; level < kWideLevels && start < end; ++level) {
-        wide_level_nodes(bin, wide, tris, queue, ctr, start, end, m, node_cap, tri_cap, bin_internal, status, s_box,
-                         s_ref, choice);
+        wide_level_nodes(bin, wide, tris, queue, ctr, start, end, m, node_cap, tri_cap, bin_internal, status,
+                         s_stage, choice);
         grid.sync();
         const uint32_t next = __ldcg(&ctr[0]);  // every node allocated so far: final after the barrier
         grid.sync();
@@ -643,8 +709,7 @@ __global__ void k_wide_init_batch(WideBatch wb)
 // sizes. Block 0 moves every tree to its next level between the two barriers.
 __global__ void __launch_bounds__(kWideBlock) k_wide_levels_batch(WideBatch wb)
 {
-    __shared__ float s_box[8 * 6][kWideBlock];
-    __shared__ uint32_t s_ref[8][kWideBlock];
+    __shared__ WideStage s_stage;
     __shared__ uint32_t s_start[kWideBatchMax], s_end[kWideBatchMax], s_rot[kWideBatchMax + 1];
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
     const uint32_t n = min(wb.count, kWideBatchMax);
@@ -672,7 +737,7 @@ __global__ void __launch_bounds__(kWideBlock) k_wide_levels_batch(WideBatch wb)
             const WideBatchTree& T = wb.t[i];
             wide_level_nodes(T.bin, T.wide, T.tris, T.queue, T.ctr, s_start[i], s_end[i],
                              __uint_as_float(__ldcg(&T.ctr[3])), T.node_cap, T.tri_cap, T.bin_internal, T.status,
-                             s_box, s_ref, nullptr, s_rot[i]);
+                             s_stage, nullptr, s_rot[i]);
         }
         grid.sync();
         if (blockIdx.x == 0 && threadIdx.x < n) {  // every node allocated so far: final after the barrier
