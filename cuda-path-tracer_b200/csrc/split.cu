@@ -19,9 +19,10 @@
 // Steps (all on the device, one stream, the piece count never leaves the GPU):
 //   k_split_weight/total  w_i = sqrt(max(0, area(box_i) - 2 area(tri_i))), sum in fixed order
 //   k_split_count         pieces s_i = 1 + min(63, floor(extra * w_i / sum w)) -> sum s_i <= n + extra
-//   k_split_scan_tiles    piece offsets of each 4096-triangle tile, total piece count
-//   k_split_first         each triangle's first piece (exclusive offsets, in place of the counts)
-//   k_split_emit          pieces, 64 per thread (balanced however the triangles are cut):
+//   k_split_scan_tiles    piece offsets of each 1024-triangle tile, total piece count
+//   k_split_first         each triangle's first piece (exclusive offsets, in place of the counts),
+//                         every fourth piece's triangle
+//   k_split_emit          pieces, 4 per thread (balanced however the triangles are cut):
 //                         clipped boxes, Morton keys of their centres in the root box,
 //                         digit histograms, zeroed look-back state
 //   k_scan_offsets, k_onesweep x P, k_topology   as the main build, on the device count
@@ -42,8 +43,8 @@ namespace {
 
 constexpr int kSplitBlock = 256;
 constexpr int kMaxPieces = 64;
-constexpr int kScanItems = 16;
-constexpr int kScanTile = kSplitBlock * kScanItems;  // triangles per emit / count tile
+constexpr int kScanItems = 4;
+constexpr int kScanTile = kSplitBlock * kScanItems;  // triangles per count tile
 constexpr int kWeightBlocks = 1024;
 
 __device__ __forceinline__ void tri_box(const cpt_triangle& t, float lo[3], float hi[3])
@@ -94,11 +95,19 @@ __global__ void __launch_bounds__(kSplitBlock) k_split_weight(const cpt_triangle
     if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
 
-__global__ void k_split_total(const double* __restrict__ partial, int blocks, double* __restrict__ total)
+// The partial sums in block order: one thread adds them (the order is part of the result),
+// from shared memory, where every thread has put one (1024 dependent loads from device
+// memory took 40 us, 4 now).
+__global__ void __launch_bounds__(kWeightBlocks) k_split_total(const double* __restrict__ partial,
+                                                               double* __restrict__ total)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ double s_part[kWeightBlocks];
+    s_part[threadIdx.x] = partial[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     double t = 0.0;
-    for (int b = 0; b < blocks; ++b) t += partial[b];
+#pragma unroll 16
+    for (int b = 0; b < kWeightBlocks; ++b) t += s_part[b];
     *total = t;
 }
 
@@ -146,11 +155,10 @@ __global__ void __launch_bounds__(kSplitBlock) k_split_count(const cpt_triangle*
                                                              uint32_t* __restrict__ tile_sums)
 {
     const double tot = *total;
-    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t sum = 0;
-#pragma unroll 4
+#pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        const uint32_t i = base + k;
+        const uint32_t i = blockIdx.x * kScanTile + k * kSplitBlock + threadIdx.x;
         if (i >= n) break;
         const uint32_t c = piece_count(tris[i], tot, extra);
         counts[i] = c;
@@ -166,30 +174,35 @@ __global__ void __launch_bounds__(1024) k_split_scan_tiles(uint32_t* __restrict_
                                                            uint32_t capacity, uint32_t* __restrict__ n_pieces,
                                                            uint32_t* __restrict__ status)
 {
-    __shared__ uint32_t s_part[1024];
-    const int per = (int)((tiles + 1023) / 1024);
+    __shared__ uint32_t s_warp[32];
+    const int per = (int)((tiles + 1023) / 1024), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t loc = 0;
     for (int k = 0; k < per; ++k) {
         const uint32_t t = threadIdx.x * per + k;
         if (t < tiles) loc += tile_sums[t];
     }
-    s_part[threadIdx.x] = loc;
+    auto warp_scan = [&](uint32_t x) {  // inclusive
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        return x;
+    };
+    const uint32_t x = warp_scan(loc);
+    if (lane == 31) s_warp[warp] = x;
     __syncthreads();
+    if (warp == 0) s_warp[lane] = warp_scan(s_warp[lane]);
+    __syncthreads();
+    uint32_t run = (warp ? s_warp[warp - 1] : 0u) + x - loc;
     if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int k = 0; k < 1024; ++k) {
-            const uint32_t v = s_part[k];
-            s_part[k] = run;
-            run += v;
-        }
-        if (run > capacity) {  // cannot happen (the shares sum to at most `extra`); stay in bounds
+        uint32_t all = s_warp[31];
+        if (all > capacity) {  // cannot happen (the shares sum to at most `extra`); stay in bounds
             atomicOr(status, CPT_STATUS_BAD_INDEX);
-            run = capacity;
+            all = capacity;
         }
-        *n_pieces = run;
+        *n_pieces = all;
     }
-    __syncthreads();
-    uint32_t run = s_part[threadIdx.x];
     for (int k = 0; k < per; ++k) {
         const uint32_t t = threadIdx.x * per + k;
         if (t < tiles) {
@@ -200,61 +213,90 @@ __global__ void __launch_bounds__(1024) k_split_scan_tiles(uint32_t* __restrict_
     }
 }
 
-// Box of triangle t clipped to lo_s <= x_axis <= hi_s (conservative, see the file comment).
+// Box of triangle t clipped to lo_s <= x_axis <= hi_s (conservative, see the file comment):
+// Sutherland-Hodgman against x >= lo_s, then x <= hi_s. The first clip leaves up to four of
+// six possible points (each corner, and after it the cut of the edge that leaves it); the
+// second only needs each point's successor and the extent of what remains, so it runs over
+// the six from the last to the first with the successor carried along, all in registers
+// (an array of points in local memory, indexed at run time, took 3 x as long).
 __device__ __forceinline__ void clip_box(const cpt_triangle& t, int axis, float lo_s, float hi_s, const float tlo[3],
                                          const float thi[3], float bmn[3], float bmx[3])
 {
-    float poly[5][3], tmp[5][3];
-    int np = 3;
+    const float v[3][3] = {{t.v0[0], t.v0[1], t.v0[2]}, {t.v1[0], t.v1[1], t.v1[2]}, {t.v2[0], t.v2[1], t.v2[2]}};
+    auto along = [&](const float (&p)[3]) { return axis == 0 ? p[0] : axis == 1 ? p[1] : p[2]; };
+    float pt[6][3];
+    bool have[6];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) { poly[0][a] = t.v0[a]; poly[1][a] = t.v1[a]; poly[2][a] = t.v2[a]; }
-    // clip against x >= lo_s, then x <= hi_s (Sutherland-Hodgman)
+    for (int k = 0; k < 3; ++k) {
+        const float(&a)[3] = v[k];
+        const float(&b)[3] = v[(k + 1) % 3];
+        const float da = along(a) - lo_s, db = along(b) - lo_s;
+        const bool ina = da >= 0.f, inb = db >= 0.f;
+        const float s = da / (da - db);
+        have[2 * k] = ina;
+        have[2 * k + 1] = ina != inb;
 #pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        const float plane = side == 0 ? lo_s : hi_s;
-        int nt = 0;
-        for (int k = 0; k < np; ++k) {
-            const float* a = poly[k];
-            const float* b = poly[(k + 1) % np];
-            const float da = side == 0 ? a[axis] - plane : plane - a[axis];
-            const float db = side == 0 ? b[axis] - plane : plane - b[axis];
-            const bool ina = da >= 0.f, inb = db >= 0.f;
-            if (ina && nt < 5) {
-                tmp[nt][0] = a[0]; tmp[nt][1] = a[1]; tmp[nt][2] = a[2];
-                ++nt;
-            }
-            if (ina != inb && nt < 5) {
-                const float s = da / (da - db);
+        for (int c = 0; c < 3; ++c) {
+            pt[2 * k][c] = a[c];
+            pt[2 * k + 1][c] = a[c] + s * (b[c] - a[c]);
+        }
+    }
+    float nx[3] = {0.f, 0.f, 0.f};  // the successor of the last point: the first one there is
 #pragma unroll
-                for (int c = 0; c < 3; ++c) tmp[nt][c] = a[c] + s * (b[c] - a[c]);
-                ++nt;
+    for (int k = 5; k >= 0; --k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) nx[c] = have[k] ? pt[k][c] : nx[c];
+    float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    bool any = false;
+#pragma unroll
+    for (int k = 5; k >= 0; --k) {
+        if (!have[k]) continue;
+        const float(&a)[3] = pt[k];
+        const float da = hi_s - along(a), db = hi_s - along(nx);
+        const bool ina = da >= 0.f, inb = db >= 0.f;
+        any = any || ina || inb;
+        if (ina)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { mn[c] = fminf(mn[c], a[c]); mx[c] = fmaxf(mx[c], a[c]); }
+        if (ina != inb) {
+            const float s = da / (da - db);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float x = a[c] + s * (nx[c] - a[c]);
+                mn[c] = fminf(mn[c], x);
+                mx[c] = fmaxf(mx[c], x);
             }
         }
-        np = nt;
-        for (int k = 0; k < np; ++k)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) poly[k][c] = tmp[k][c];
+        for (int c = 0; c < 3; ++c) nx[c] = a[c];
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) { bmn[a] = tlo[a]; bmx[a] = thi[a]; }
-    if (np > 0) {
+    if (any) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            float mn = poly[0][a], mx = poly[0][a];
-            for (int k = 1; k < np; ++k) { mn = fminf(mn, poly[k][a]); mx = fmaxf(mx, poly[k][a]); }
-            const float eps = (fabsf(mn) + fabsf(mx) + (thi[a] - tlo[a])) * 9.5367431640625e-07f;  // 2^-20
-            bmn[a] = fmaxf(mn - eps, tlo[a]);
-            bmx[a] = fminf(mx + eps, thi[a]);
+            const float eps = (fabsf(mn[a]) + fabsf(mx[a]) + (thi[a] - tlo[a])) * 9.5367431640625e-07f;  // 2^-20
+            bmn[a] = fmaxf(mn[a] - eps, tlo[a]);
+            bmx[a] = fminf(mx[a] + eps, thi[a]);
         }
     }
-    bmn[axis] = fmaxf(lo_s, tlo[axis]);
-    bmx[axis] = fminf(hi_s, thi[axis]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (a == axis) {
+            bmn[a] = fmaxf(lo_s, tlo[a]);
+            bmx[a] = fminf(hi_s, thi[a]);
+        }
 }
 
+// Pieces per thread of k_split_emit.
+constexpr int kEmitPieces = 4;
+
 // Piece counts -> exclusive per-triangle piece offsets, in place (tile offsets from
-// k_split_scan_tiles, a block scan inside the tile).
+// k_split_scan_tiles, a block scan inside the tile). owner[j / kEmitPieces]: the triangle of
+// piece j, for every multiple j of kEmitPieces (where the emitting threads start).
 __global__ void __launch_bounds__(kSplitBlock) k_split_first(uint32_t n, uint32_t* __restrict__ counts,
-                                                             const uint32_t* __restrict__ tile_offsets)
+                                                             const uint32_t* __restrict__ tile_offsets,
+                                                             uint32_t* __restrict__ owner, uint32_t capacity)
 {
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t c[kScanItems];
@@ -271,20 +313,23 @@ __global__ void __launch_bounds__(kSplitBlock) k_split_first(uint32_t n, uint32_
     for (int k = 0; k < kScanItems; ++k) {
         const uint32_t i = base + k;
         if (i < n) counts[i] = off;
+        for (uint32_t j = (off + kEmitPieces - 1) / kEmitPieces; j * kEmitPieces < off + c[k]; ++j)
+            if (j * kEmitPieces < capacity) owner[j] = i;
         off += c[k];
     }
 }
 
 // Pieces of the triangles, kEmitPieces consecutive pieces per thread whatever the
-// triangles they come from (a long hairball triangle is cut into up to 64 pieces):
-// piece j belongs to the triangle i with first[i] <= j < first[i + 1], found once per
-// thread by binary search. Writes the piece box, its Morton key and all the digit
-// histograms of the sort, and zeroes the sort's look-back state.
-constexpr int kEmitPieces = 64;
-
+// triangles they come from (a long hairball triangle is cut into up to 64 pieces); the
+// first one's triangle comes from owner. Writes the piece box, its Morton key and all the
+// digit histograms of the sort, and zeroes the sort's look-back state. 11.8 M pieces:
+// 64 pieces per thread after a binary search, clipping in local memory, 1,475 us (15 % of
+// the warps resident; 355 us for the 100,000 of a small scene); now 348 us
+// and 15 (4, 8 and 16 pieces per thread are within 2 %).
 template <typename K>
-__global__ void __launch_bounds__(kSplitBlock) k_split_emit(const cpt_triangle* __restrict__ tris, uint32_t n,
+__global__ void __launch_bounds__(kSplitBlock, 4) k_split_emit(const cpt_triangle* __restrict__ tris, uint32_t n,
                                                             const uint32_t* __restrict__ first,
+                                                            const uint32_t* __restrict__ owner,
                                                             const uint32_t* __restrict__ n_pieces,
                                                             const cpt_bbox* __restrict__ root,
                                                             float4* __restrict__ pieces, K* __restrict__ keys,
@@ -310,13 +355,7 @@ __global__ void __launch_bounds__(kSplitBlock) k_split_emit(const cpt_triangle* 
     const uint32_t np = *n_pieces;
     const uint64_t j0 = ((uint64_t)blockIdx.x * kSplitBlock + threadIdx.x) * kEmitPieces;
     if (j0 < np) {
-        uint32_t lo = 0, hi = n - 1;  // the last triangle whose first piece is at or before j0
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (first[mid] <= j0) lo = mid;
-            else hi = mid - 1;
-        }
-        uint32_t i = lo;
+        uint32_t i = min(owner[j0 / kEmitPieces], n - 1);
         uint32_t fi = first[i];
         uint32_t ei = i + 1 < n ? first[i + 1] : np;
         cpt_triangle t = tris[i];
@@ -346,8 +385,10 @@ __global__ void __launch_bounds__(kSplitBlock) k_split_emit(const cpt_triangle* 
 #pragma unroll
                 for (int a = 0; a < 3; ++a) { bmn[a] = tlo[a]; bmx[a] = thi[a]; }
             } else {
-                const float lo_s = p == 0 ? tlo[axis] : tlo[axis] + ext * ((float)p / (float)s);
-                const float hi_s = p + 1 == s ? thi[axis] : tlo[axis] + ext * ((float)(p + 1) / (float)s);
+                const float la = axis == 0 ? tlo[0] : axis == 1 ? tlo[1] : tlo[2];
+                const float ha = axis == 0 ? thi[0] : axis == 1 ? thi[1] : thi[2];
+                const float lo_s = p == 0 ? la : la + ext * ((float)p / (float)s);
+                const float hi_s = p + 1 == s ? ha : la + ext * ((float)(p + 1) / (float)s);
                 clip_box(t, axis, lo_s, hi_s, tlo, thi, bmn, bmx);
             }
             pieces[2 * (size_t)j] = make_float4(bmn[0], bmn[1], bmn[2], __uint_as_float(i));
@@ -1011,17 +1052,18 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
     CPT_CUDA_TRY(cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * P * kRadix, stream));
     k_split_weight<<<kWeightBlocks, kSplitBlock, 0, stream>>>(bvh->tris, n, s.partial);
     CPT_LAUNCH_CHECK();
-    k_split_total<<<1, 32, 0, stream>>>(s.partial, kWeightBlocks, s.total);
+    k_split_total<<<1, kWeightBlocks, 0, stream>>>(s.partial, s.total);
     CPT_LAUNCH_CHECK();
     k_split_count<<<ctiles, kSplitBlock, 0, stream>>>(bvh->tris, n, s.total, extra, s.counts, s.tile_sums);
     CPT_LAUNCH_CHECK();
     k_split_scan_tiles<<<1, 1024, 0, stream>>>(s.tile_sums, ctiles, cap, s.n_pieces, bvh->status);
     CPT_LAUNCH_CHECK();
-    k_split_first<<<ctiles, kSplitBlock, 0, stream>>>(n, s.counts, s.tile_sums);
+    uint32_t* owner = s.children;  // (free until the topology is built)
+    k_split_first<<<ctiles, kSplitBlock, 0, stream>>>(n, s.counts, s.tile_sums, owner, cap);
     CPT_LAUNCH_CHECK();
     const uint32_t eblocks = (uint32_t)(((uint64_t)cap + (uint64_t)kSplitBlock * kEmitPieces - 1) /
                                         ((uint64_t)kSplitBlock * kEmitPieces));
-    k_split_emit<K><<<eblocks, kSplitBlock, 0, stream>>>(bvh->tris, n, s.counts, s.n_pieces, bvh->node_boxes,
+    k_split_emit<K><<<eblocks, kSplitBlock, 0, stream>>>(bvh->tris, n, s.counts, owner, s.n_pieces, bvh->node_boxes,
                                                          s.pieces, s.keys[0], s.hist, s.zero, s.zero_words);
     CPT_LAUNCH_CHECK();
     k_scan_offsets<<<P, kRadix, 0, stream>>>(s.hist, s.offsets);
