@@ -264,8 +264,6 @@ struct SortScratch {
     float* tris_copy;
 };
 
-inline uint32_t num_tiles(uint32_t n) { return (n + kSortTile - 1) / kSortTile; }
-
 template <typename K>
 size_t scratch_layout(uint32_t n, void* base, SortScratch<K>* s)
 {
@@ -277,11 +275,13 @@ size_t scratch_layout(uint32_t n, void* base, SortScratch<K>* s)
     t.vals[1] = c.take<uint32_t>(n);
     t.hist = c.take<uint32_t>((size_t)P * kRadix);
     t.offsets = c.take<uint32_t>((size_t)P * kRadix);
-    t.zero_words = 32 + (size_t)P * num_tiles(n) * kRadix;
-    t.zero_region = c.take<uint32_t>(t.zero_words);
+    t.zero_words = sort_zero_words(n, P);
+    t.zero_region = c.take<uint32_t>(sort_zero_reserve(n, P));
     t.tile_counters = t.zero_region;
     t.lookback = t.zero_region ? t.zero_region + 32 : nullptr;
-    t.counters = c.take<int>(n);
+    // the tree's words, one per split: in the look-back region (free after the sort) where it
+    // holds them, as it does under the smaller sort tiles
+    t.counters = sort_zero_reserve(n, P) - 32 >= n ? reinterpret_cast<int*>(t.lookback) : c.take<int>(n);
     t.bounds_partial = c.take<float>(6 * kBoundsBlocks);
     t.dev_box = c.take<float>(8);
     t.tris_copy = c.take<float>(10ull * n);
@@ -304,30 +304,21 @@ int sort_keys(const SortScratch<K>& s, uint32_t n, K* keys, uint32_t* status, So
                                       true, stream);
     } else {
         constexpr int P = KeyTraits<K>::passes;
-        const uint32_t tiles = num_tiles(n);
-        const size_t smem = onesweep_smem<K>();
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const uint32_t tiles = sort_tiles(n);
         K* kbuf[2] = {keys, s.keys_alt};
         for (int p = 0; p < P; ++p) {
             const K* kin = kbuf[p & 1];
             K* kout = kbuf[(p + 1) & 1];
-            const uint32_t* vin = p == 0 ? nullptr : s.vals[(p + 1) & 1];
-            uint32_t* vout = s.vals[p & 1];
             uint32_t* lb = s.lookback + (size_t)p * tiles * kRadix;
+            SortWait w = wait;
+            if (p) w.withhold_tile0 = 0;  // (the test hook stalls the first pass only)
             CPT_PROF(K_ONESWEEP, stream);
-            if (p == 0)
-                k_onesweep<K, true><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, n, nullptr, 8 * p,
-                                                                         s.offsets + p * kRadix,
-                                                                         lb, s.tile_counters + p, status, wait);
-            else {
-                SortWait later = wait;
-                later.withhold_tile0 = 0;  // (the test hook stalls the first pass only)
-                k_onesweep<K, false><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, n, nullptr, 8 * p,
-                                                                          s.offsets + p * kRadix,
-                                                                          lb, s.tile_counters + p, status, later);
-            }
-            CPT_LAUNCH_CHECK();
+            const int rc = p == 0 ? onesweep_launch<K, true>(kin, nullptr, kout, s.vals[0], n, n, nullptr, 0, s.offsets,
+                                                             lb, s.tile_counters, status, w, stream)
+                                  : onesweep_launch<K, false>(kin, s.vals[(p + 1) & 1], kout, s.vals[p & 1], n, n,
+                                                              nullptr, 8 * p, s.offsets + p * kRadix, lb,
+                                                              s.tile_counters + p, status, w, stream);
+            if (rc) return rc;
         }
         return CPT_OK;
     }

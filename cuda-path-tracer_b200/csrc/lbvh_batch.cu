@@ -205,7 +205,6 @@ size_t batch_layout(uint64_t total, uint32_t scenes, void* base, BatchScratch<K>
     constexpr int P = KeyTraits<K>::passes;
     Carver c(base);
     BatchScratch<K> s;
-    const size_t tiles = (size_t)((total + kSortTile - 1) / kSortTile);
     for (int k = 0; k < 3; ++k) s.keys[k] = c.take<K>(total);
     s.vals[0] = c.take<uint32_t>(total);
     s.vals[1] = c.take<uint32_t>(total);
@@ -213,8 +212,8 @@ size_t batch_layout(uint64_t total, uint32_t scenes, void* base, BatchScratch<K>
     s.sid[1] = c.take<uint32_t>(total);
     s.hist = c.take<uint32_t>((size_t)(P + 1) * kRadix);
     s.offsets = c.take<uint32_t>((size_t)(P + 1) * kRadix);
-    s.zero_words = 32 + (size_t)(P + 1) * tiles * kRadix;
-    s.zero = c.take<uint32_t>(s.zero_words);
+    s.zero_words = sort_zero_words(total, P + 1);
+    s.zero = c.take<uint32_t>(sort_zero_reserve(total, P + 1));
     s.counters = c.take<int>(total - scenes);
     s.status = c.take<uint32_t>(4);
     s.tris_copy = c.take<float>(10ull * total);
@@ -252,7 +251,7 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
         k_scan_offsets<<<P + 1, kRadix, 0, stream>>>(s.hist, s.offsets);
     }
     CPT_LAUNCH_CHECK();
-    const uint32_t tiles = (bt.total + kSortTile - 1) / kSortTile;
+    const uint32_t tiles = sort_tiles(bt.total);
     uint32_t* lookback = s.zero + 32;
     if constexpr (sizeof(K) == 8) {
         // as 32-bit halves (in keys[1]); only the order is needed, k_batch_keys gathers
@@ -263,9 +262,6 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
                                                   true, stream))
             return rc;
     } else {
-        const size_t smem = onesweep_smem<K>();
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         // key passes: keys[0] -> keys[1] -> keys[2] -> keys[1] ...; values 0 -> 1 -> 0 ...
         for (int p = 0; p < P; ++p) {
             const K* kin = p == 0 ? s.keys[0] : s.keys[1 + ((p + 1) & 1)];
@@ -274,32 +270,27 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
             uint32_t* vout = s.vals[p & 1];
             uint32_t* lb = lookback + (size_t)p * tiles * kRadix;
             CPT_PROF(K_ONESWEEP, stream);
-            if (p == 0)
-                k_onesweep<K, true><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, bt.total, nullptr, 8 * p,
-                                                                         s.offsets + p * kRadix, lb, s.zero + p,
-                                                                         s.status);
-            else
-                k_onesweep<K, false><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, bt.total, nullptr,
-                                                                          8 * p, s.offsets + p * kRadix, lb,
-                                                                          s.zero + p, s.status);
-            CPT_LAUNCH_CHECK();
+            const int rc = p == 0 ? onesweep_launch<K, true>(kin, vin, kout, vout, bt.total, bt.total, nullptr, 0,
+                                                             s.offsets, lb, s.zero, s.status, SortWait(), stream)
+                                  : onesweep_launch<K, false>(kin, vin, kout, vout, bt.total, bt.total, nullptr, 8 * p,
+                                                              s.offsets + p * kRadix, lb, s.zero + p, s.status,
+                                                              SortWait(), stream);
+            if (rc) return rc;
         }
     }
     const uint32_t* order = s.vals[(P - 1) & 1];
     if (bt.scenes > 1) {  // the scene digit: one more stable pass
         k_batch_scene_ids<<<grid, kBatchBlock, 0, stream>>>(bt, order, s.sid[0]);
         CPT_LAUNCH_CHECK();
-        const size_t smem32 = onesweep_smem<uint32_t>();
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<uint32_t, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem32));
         uint32_t* vout = s.vals[P & 1];
         {
             CPT_PROF(K_ONESWEEP, stream);
-            k_onesweep<uint32_t, false><<<tiles, kSortBlock, smem32, stream>>>(
-                s.sid[0], order, s.sid[1], vout, bt.total, nullptr, 0, s.offsets + P * kRadix,
-                lookback + (size_t)P * tiles * kRadix, s.zero + P, s.status);
+            if (const int rc = onesweep_launch<uint32_t, false>(s.sid[0], order, s.sid[1], vout, bt.total, bt.total,
+                                                                nullptr, 0, s.offsets + P * kRadix,
+                                                                lookback + (size_t)P * tiles * kRadix, s.zero + P,
+                                                                s.status, SortWait(), stream))
+                return rc;
         }
-        CPT_LAUNCH_CHECK();
         order = vout;
     }
     k_batch_keys<K><<<grid, kBatchBlock, 0, stream>>>(bt, s.keys[0], order);

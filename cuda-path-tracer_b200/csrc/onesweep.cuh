@@ -14,14 +14,34 @@ namespace cpt {
 constexpr int kRadix = 256;
 constexpr int kSortBlock = 256;  // one thread per digit in the per-tile digit work
 constexpr int kSortWarps = kSortBlock / 32;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortBlock * kSortItems;  // 4096 keys per tile
+// Keys per thread of a tile. Tiles of 16 x 256 keys are the fastest once they fill the chip
+// (three to an SM, 1.8 M keys to a round); below that a pass lasts as long as one tile's chain
+// of 16 rankings while SMs wait, so smaller inputs take smaller tiles. The sort of a build,
+// with 16 / 8 / 4 keys per thread: 65,538 30-bit keys 62 / 51 / 46 us; 100,000 63-bit keys 133 /
+// 103 / 101; 200,000 135 / 107 / 119; 700,000 186 / 172 / 202; 1.05 M 200 / 237 / 257; 5.24 M 630 /
+// 677 / 851. (The smallest tiles' look-back words, 1 KB each and pass, end at 98,304 keys so
+// that the static build's scratch holds any size it takes.)
+constexpr uint32_t kSortSmall = 98304, kSortMedium = 786432;
+inline int sort_items(uint64_t n) { return n <= kSortSmall ? 4 : n <= kSortMedium ? 8 : 16; }
+inline uint32_t sort_tile(uint64_t n) { return (uint32_t)(kSortBlock * sort_items(n)); }
+inline uint32_t sort_tiles(uint64_t n) { return (uint32_t)((n + sort_tile(n) - 1) / sort_tile(n)); }
 constexpr uint32_t kFlagAgg = 1u << 30, kFlagInc = 2u << 30, kValueMask = (1u << 30) - 1;
 constexpr uint32_t kLookbackPolls = 1u << 22;  // default poll limit of one tile's look-back
 #ifndef CPT_LOOKBACK_WINDOW
 #define CPT_LOOKBACK_WINDOW 4
 #endif
 constexpr int kLookbackWindow = CPT_LOOKBACK_WINDOW;  // predecessor words read per look-back round
+
+// Words of the tile counters (32) and look-back of a sort of n, and those to reserve: never
+// fewer than for a smaller n, so that scratch sized for one count serves every smaller one.
+inline size_t sort_zero_words(uint64_t n, int passes) { return 32 + (size_t)passes * sort_tiles(n) * kRadix; }
+inline size_t sort_zero_reserve(uint64_t n, int passes)
+{
+    size_t w = sort_zero_words(n, passes);
+    for (const uint64_t edge : {(uint64_t)kSortSmall, (uint64_t)kSortMedium})
+        if (n > edge) w = w > sort_zero_words(edge, passes) ? w : sort_zero_words(edge, passes);
+    return w;
+}
 
 // Look-back wait settings of one digit pass: the poll limit, and (a test of the
 // failure path only) whether the pass's tile 0 withholds its published counts, so
@@ -65,7 +85,10 @@ __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *rei
 __device__ __forceinline__ void st_volatile(uint32_t* p, uint32_t v) { *reinterpret_cast<volatile uint32_t*>(p) = v; }
 
 template <typename K>
-constexpr size_t onesweep_smem() { return (size_t)kSortTile * sizeof(K) + (size_t)kSortTile * 4 + (size_t)kSortWarps * kRadix * 4 + 2 * kRadix * 4; }
+inline size_t onesweep_smem(int items)
+{
+    return (size_t)kSortBlock * items * (sizeof(K) + 4) + (size_t)kSortWarps * kRadix * 4 + 2 * kRadix * 4;
+}
 
 // Where a pass takes its (key, value) pairs from.
 //   kSrcKeys    key = kin[i], value = vin[i]
@@ -99,7 +122,7 @@ constexpr int onesweep_min_blocks() { return sizeof(K) == 4 ? CPT_SORT32_MIN_BLO
 // block starts (one read, shared by the block) and returns at once after a timeout,
 // like the kernels that follow the sort. A gathered value is clamped into [0, n)
 // before it indexes g64 all the same.
-template <typename K, int kSrc>
+template <typename K, int kSrc, int kItems>
 __device__ __forceinline__ void onesweep_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                                               const uint64_t* __restrict__ g64, K* __restrict__ kout,
                                               uint32_t* __restrict__ vout, uint32_t n_arg,
@@ -110,6 +133,7 @@ __device__ __forceinline__ void onesweep_pass(const K* __restrict__ kin, const u
 {
     static_assert(kSrc == kSrcKeys || kSrc == kSrcIndex || sizeof(K) == (kSrc == kSrcFull64 ? 8 : 4),
                   "64-bit sources give 32-bit halves or whole 64-bit keys");
+    constexpr int kSortItems = kItems, kSortTile = kSortBlock * kItems;
     extern __shared__ __align__(16) unsigned char smem[];
     K* s_keys = reinterpret_cast<K*>(smem);
     uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + kSortTile);
@@ -263,7 +287,7 @@ __device__ __forceinline__ void onesweep_pass(const K* __restrict__ kin, const u
 #endif
 
 // One digit pass over (key, value) pairs; kFirst: the values are the element indices.
-template <typename K, bool kFirst>
+template <typename K, bool kFirst, int kItems>
 __global__ void __launch_bounds__(kSortBlock, CPT_SORT_MIN_BLOCKS) k_onesweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                          K* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n_arg,
                                                          const uint32_t* __restrict__ n_ptr,
@@ -272,20 +296,20 @@ __global__ void __launch_bounds__(kSortBlock, CPT_SORT_MIN_BLOCKS) k_onesweep(co
                                                          uint32_t* __restrict__ tile_counter,
                                                          uint32_t* __restrict__ status, SortWait wait = SortWait())
 {
-    onesweep_pass<K, kFirst ? kSrcIndex : kSrcKeys>(kin, vin, nullptr, kout, vout, n_arg, n_ptr, shift, offsets,
+    onesweep_pass<K, kFirst ? kSrcIndex : kSrcKeys, kItems>(kin, vin, nullptr, kout, vout, n_arg, n_ptr, shift, offsets,
                                                     lookback, tile_counter, status, wait);
 }
 
 // One digit pass of a 64-bit key sort done as two 32-bit halves (kSrcLow64,
 // kSrcKeys over the halves, kSrcHigh64, kSrcFull64).
-template <typename K, int kSrc>
+template <typename K, int kSrc, int kItems>
 __global__ void __launch_bounds__(kSortBlock, onesweep_min_blocks<K>()) k_onesweep_halves(
     const K* __restrict__ kin, const uint32_t* __restrict__ vin, const uint64_t* __restrict__ g64,
     K* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n_arg, const uint32_t* __restrict__ n_ptr,
     int shift, const uint32_t* __restrict__ offsets, uint32_t* __restrict__ lookback,
     uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ status, SortWait wait)
 {
-    onesweep_pass<K, kSrc>(kin, vin, g64, kout, vout, n_arg, n_ptr, shift, offsets, lookback, tile_counter, status,
+    onesweep_pass<K, kSrc, kItems>(kin, vin, g64, kout, vout, n_arg, n_ptr, shift, offsets, lookback, tile_counter, status,
                            wait);
 }
 
@@ -298,21 +322,22 @@ __global__ void __launch_bounds__(kSortBlock, onesweep_min_blocks<K>()) k_oneswe
 // is n, or *n_ptr on the device (cap bounds it and sizes the grids). offsets: the
 // 8 x 256 digit offsets; lookback: 8 regions of tiles x 256 words, tile_counters: 8
 // words, all zeroed. prof: each pass timed as K_ONESWEEP.
-inline int onesweep_sort64_halves(const uint64_t* keys_in, uint64_t* keys_out, uint32_t cap, uint32_t n,
+template <int kItems>
+inline int onesweep_sort64_halves_t(const uint64_t* keys_in, uint64_t* keys_out, uint32_t cap, uint32_t n,
                                   const uint32_t* n_ptr, uint32_t* const vals[2], const uint32_t* offsets,
                                   uint32_t* lookback, uint32_t* tile_counters, uint32_t* status, SortWait wait,
                                   bool whole_keys, bool prof, cudaStream_t stream)
 {
     constexpr int P = 8;
-    const uint32_t tiles = (cap + kSortTile - 1) / kSortTile;
-    const size_t smem32 = onesweep_smem<uint32_t>(), smem64 = onesweep_smem<uint64_t>();
-    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint32_t, kSrcLow64>,
+    const uint32_t tiles = sort_tiles(cap);
+    const size_t smem32 = onesweep_smem<uint32_t>(kItems), smem64 = onesweep_smem<uint64_t>(kItems);
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint32_t, kSrcLow64, kItems>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem32));
-    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint32_t, kSrcKeys>,
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint32_t, kSrcKeys, kItems>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem32));
-    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint32_t, kSrcHigh64>,
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint32_t, kSrcHigh64, kItems>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem32));
-    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint64_t, kSrcFull64>,
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep_halves<uint64_t, kSrcFull64, kItems>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64));
     uint32_t* half[2] = {reinterpret_cast<uint32_t*>(keys_out), reinterpret_cast<uint32_t*>(keys_out) + cap};
     for (int p = 0; p < P; ++p) {
@@ -324,16 +349,16 @@ inline int onesweep_sort64_halves(const uint64_t* keys_in, uint64_t* keys_out, u
         if (p) w.withhold_tile0 = 0;  // (the test hook stalls the first pass only)
         auto launch = [&]() {
             if (p == 0)
-                k_onesweep_halves<uint32_t, kSrcLow64><<<tiles, kSortBlock, smem32, stream>>>(
+                k_onesweep_halves<uint32_t, kSrcLow64, kItems><<<tiles, kSortBlock, smem32, stream>>>(
                     nullptr, nullptr, keys_in, half[0], vout, n, n_ptr, 0, off, lb, tile_counters + p, status, w);
             else if (p == 4)
-                k_onesweep_halves<uint32_t, kSrcHigh64><<<tiles, kSortBlock, smem32, stream>>>(
+                k_onesweep_halves<uint32_t, kSrcHigh64, kItems><<<tiles, kSortBlock, smem32, stream>>>(
                     nullptr, vin, keys_in, half[0], vout, n, n_ptr, 0, off, lb, tile_counters + p, status, w);
             else if (p == P - 1 && whole_keys)
-                k_onesweep_halves<uint64_t, kSrcFull64><<<tiles, kSortBlock, smem64, stream>>>(
+                k_onesweep_halves<uint64_t, kSrcFull64, kItems><<<tiles, kSortBlock, smem64, stream>>>(
                     nullptr, vin, keys_in, keys_out, vout, n, n_ptr, 8 * p, off, lb, tile_counters + p, status, w);
             else
-                k_onesweep_halves<uint32_t, kSrcKeys><<<tiles, kSortBlock, smem32, stream>>>(
+                k_onesweep_halves<uint32_t, kSrcKeys, kItems><<<tiles, kSortBlock, smem32, stream>>>(
                     half[(p + 1) & 1], vin, nullptr, half[p & 1], vout, n, n_ptr, 8 * (p & 3), off, lb,
                     tile_counters + p, status, w);
         };
@@ -348,5 +373,50 @@ inline int onesweep_sort64_halves(const uint64_t* keys_in, uint64_t* keys_out, u
     return CPT_OK;
 }
 
+inline int onesweep_sort64_halves(const uint64_t* keys_in, uint64_t* keys_out, uint32_t cap, uint32_t n,
+                                  const uint32_t* n_ptr, uint32_t* const vals[2], const uint32_t* offsets,
+                                  uint32_t* lookback, uint32_t* tile_counters, uint32_t* status, SortWait wait,
+                                  bool whole_keys, bool prof, cudaStream_t stream)
+{
+    switch (sort_items(cap)) {
+    case 4: return onesweep_sort64_halves_t<4>(keys_in, keys_out, cap, n, n_ptr, vals, offsets, lookback,
+                                               tile_counters, status, wait, whole_keys, prof, stream);
+    case 8: return onesweep_sort64_halves_t<8>(keys_in, keys_out, cap, n, n_ptr, vals, offsets, lookback,
+                                               tile_counters, status, wait, whole_keys, prof, stream);
+    default: return onesweep_sort64_halves_t<16>(keys_in, keys_out, cap, n, n_ptr, vals, offsets, lookback,
+                                                 tile_counters, status, wait, whole_keys, prof, stream);
+    }
+}
+
+// One digit pass over cap elements at most (tiles sized for cap): k_onesweep at its tile size.
+template <typename K, bool kFirst, int kItems>
+inline int onesweep_launch_t(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t cap, uint32_t n,
+                             const uint32_t* n_ptr, int shift, const uint32_t* offsets, uint32_t* lookback,
+                             uint32_t* tile_counter, uint32_t* status, SortWait wait, cudaStream_t stream)
+{
+    const size_t smem = onesweep_smem<K>(kItems);
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, kFirst, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+    k_onesweep<K, kFirst, kItems><<<sort_tiles(cap), kSortBlock, smem, stream>>>(kin, vin, kout, vout, n, n_ptr, shift,
+                                                                                 offsets, lookback, tile_counter,
+                                                                                 status, wait);
+    CPT_LAUNCH_CHECK();
+    return CPT_OK;
+}
+
+template <typename K, bool kFirst>
+inline int onesweep_launch(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t cap, uint32_t n,
+                           const uint32_t* n_ptr, int shift, const uint32_t* offsets, uint32_t* lookback,
+                           uint32_t* tile_counter, uint32_t* status, SortWait wait, cudaStream_t stream)
+{
+    switch (sort_items(cap)) {
+    case 4: return onesweep_launch_t<K, kFirst, 4>(kin, vin, kout, vout, cap, n, n_ptr, shift, offsets, lookback,
+                                                   tile_counter, status, wait, stream);
+    case 8: return onesweep_launch_t<K, kFirst, 8>(kin, vin, kout, vout, cap, n, n_ptr, shift, offsets, lookback,
+                                                   tile_counter, status, wait, stream);
+    default: return onesweep_launch_t<K, kFirst, 16>(kin, vin, kout, vout, cap, n, n_ptr, shift, offsets, lookback,
+                                                     tile_counter, status, wait, stream);
+    }
+}
 
 }  // namespace cpt

@@ -880,15 +880,14 @@ size_t render_layout(const cpt_render_params* p, uint64_t pixels, void* base, Re
         s.second = Lane{};
     }
     if (p->ray_sort) {
-        const size_t tiles = (s.capacity + kSortTile - 1) / kSortTile;
         for (int k = 0; k < 2; ++k) {
             s.sort_keys[k] = c.take<uint32_t>(s.capacity);
             s.sort_vals[k] = c.take<uint32_t>(s.capacity);
         }
         s.sort_hist = c.take<uint32_t>(kRayKeyPasses * kRadix);
         s.sort_offsets = c.take<uint32_t>(kRayKeyPasses * kRadix);
-        s.sort_zero_words = 32 + (size_t)kRayKeyPasses * tiles * kRadix;
-        s.sort_zero = c.take<uint32_t>(s.sort_zero_words);
+        s.sort_zero_words = sort_zero_words(s.capacity, kRayKeyPasses);
+        s.sort_zero = c.take<uint32_t>(sort_zero_reserve(s.capacity, kRayKeyPasses));
     } else {
         s.sort_keys[0] = s.sort_keys[1] = s.sort_vals[0] = s.sort_vals[1] = nullptr;
         s.sort_hist = s.sort_offsets = s.sort_zero = nullptr;
@@ -904,7 +903,7 @@ size_t render_layout(const cpt_render_params* p, uint64_t pixels, void* base, Re
 int sort_queue(const RenderScratch& rs, const float4* queue, const uint32_t* count, const cpt_bbox* root,
                uint32_t* status, cudaStream_t stream)
 {
-    const uint32_t tiles = (rs.capacity + kSortTile - 1) / kSortTile;
+    const uint32_t tiles = sort_tiles(rs.capacity);
     const int sms = sm_count();
     CPT_CUDA_TRY(cudaMemsetAsync(rs.sort_hist, 0, sizeof(uint32_t) * kRayKeyPasses * kRadix, stream));
     {
@@ -918,9 +917,6 @@ int sort_queue(const RenderScratch& rs, const float4* queue, const uint32_t* cou
         k_scan_offsets<<<kRayKeyPasses, kRadix, 0, stream>>>(rs.sort_hist, rs.sort_offsets);
     }
     CPT_LAUNCH_CHECK();
-    const size_t smem = onesweep_smem<uint32_t>();
-    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<uint32_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<uint32_t, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     uint32_t* lookback = rs.sort_zero + 32;
     for (int p = 0; p < kRayKeyPasses; ++p) {
         const uint32_t* kin = rs.sort_keys[p & 1];
@@ -928,17 +924,14 @@ int sort_queue(const RenderScratch& rs, const float4* queue, const uint32_t* cou
         const uint32_t* vin = p == 0 ? nullptr : rs.sort_vals[(p + 1) & 1];
         uint32_t* vout = rs.sort_vals[p & 1];
         CPT_PROF(K_RAY_SORT, stream);
-        if (p == 0)
-            k_onesweep<uint32_t, true><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, 0, count, 8 * p,
-                                                                            rs.sort_offsets + p * kRadix,
-                                                                            lookback + (size_t)p * tiles * kRadix,
-                                                                            rs.sort_zero + p, status);
-        else
-            k_onesweep<uint32_t, false><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, 0, count, 8 * p,
-                                                                             rs.sort_offsets + p * kRadix,
-                                                                             lookback + (size_t)p * tiles * kRadix,
-                                                                             rs.sort_zero + p, status);
-        CPT_LAUNCH_CHECK();
+        uint32_t* lb = lookback + (size_t)p * tiles * kRadix;
+        const int rc = p == 0 ? onesweep_launch<uint32_t, true>(kin, vin, kout, vout, rs.capacity, 0, count, 0,
+                                                                rs.sort_offsets, lb, rs.sort_zero, status, SortWait(),
+                                                                stream)
+                              : onesweep_launch<uint32_t, false>(kin, vin, kout, vout, rs.capacity, 0, count, 8 * p,
+                                                                 rs.sort_offsets + p * kRadix, lb, rs.sort_zero + p,
+                                                                 status, SortWait(), stream);
+        if (rc) return rc;
     }
     return CPT_OK;
 }

@@ -1007,7 +1007,6 @@ size_t split_layout(uint32_t n, uint32_t cap, bool treelet, void* base, SplitScr
     Carver c(base);
     SplitScratch<K> s;
     const uint32_t ctiles = (n + kScanTile - 1) / kScanTile;
-    const size_t sort_tiles = (cap + kSortTile - 1) / kSortTile;
     s.partial = c.take<double>(kWeightBlocks);
     s.total = c.take<double>(1);
     s.counts = c.take<uint32_t>(n);
@@ -1020,8 +1019,8 @@ size_t split_layout(uint32_t n, uint32_t cap, bool treelet, void* base, SplitScr
     s.vals[1] = c.take<uint32_t>(cap);
     s.hist = c.take<uint32_t>((size_t)P * kRadix);
     s.offsets = c.take<uint32_t>((size_t)P * kRadix);
-    s.zero_words = 32 + (size_t)P * sort_tiles * kRadix;
-    s.zero = c.take<uint32_t>(s.zero_words);
+    s.zero_words = sort_zero_words(cap, P);
+    s.zero = c.take<uint32_t>(sort_zero_reserve(cap, P));
     s.children = c.take<uint32_t>(cap);
     s.parents_leaf = c.take<uint32_t>(cap);
     s.parents_internal = c.take<uint32_t>(cap);
@@ -1068,7 +1067,7 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
     CPT_LAUNCH_CHECK();
     k_scan_offsets<<<P, kRadix, 0, stream>>>(s.hist, s.offsets);
     CPT_LAUNCH_CHECK();
-    const uint32_t tiles = (cap + kSortTile - 1) / kSortTile;
+    const uint32_t tiles = sort_tiles(cap);
     uint32_t* lookback = s.zero + 32;
     const K* keys;
     if constexpr (sizeof(K) == 8) {  // as 32-bit halves: the sorted keys end in keys[1]
@@ -1079,24 +1078,18 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
             return rc;
         keys = s.keys[1];
     } else {
-        const size_t smem = onesweep_smem<K>();
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         for (int p = 0; p < P; ++p) {
             const K* kin = s.keys[p & 1];
             K* kout = s.keys[(p + 1) & 1];
             const uint32_t* vin = p == 0 ? nullptr : s.vals[(p + 1) & 1];
             uint32_t* vout = s.vals[p & 1];
             uint32_t* lb = lookback + (size_t)p * tiles * kRadix;
-            if (p == 0)
-                k_onesweep<K, true><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, 0, s.n_pieces, 8 * p,
-                                                                         s.offsets + p * kRadix, lb, s.zero + p,
-                                                                         bvh->status);
-            else
-                k_onesweep<K, false><<<tiles, kSortBlock, smem, stream>>>(kin, vin, kout, vout, 0, s.n_pieces, 8 * p,
-                                                                          s.offsets + p * kRadix, lb, s.zero + p,
-                                                                          bvh->status);
-            CPT_LAUNCH_CHECK();
+            const int rc = p == 0 ? onesweep_launch<K, true>(kin, vin, kout, vout, cap, 0, s.n_pieces, 0, s.offsets, lb,
+                                                             s.zero, bvh->status, SortWait(), stream)
+                                  : onesweep_launch<K, false>(kin, vin, kout, vout, cap, 0, s.n_pieces, 8 * p,
+                                                              s.offsets + p * kRadix, lb, s.zero + p, bvh->status,
+                                                              SortWait(), stream);
+            if (rc) return rc;
         }
         keys = s.keys[P & 1];
     }
