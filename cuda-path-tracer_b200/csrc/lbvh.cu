@@ -10,9 +10,10 @@
 //   k_morton           morton_encoder (BVHBuilder.cu:12-32)    40 B tri -> K B key, digit histograms
 //   k_scan_offsets     (part of thrust::sort_by_key)           P x 256 counters
 //   k_onesweep x P     thrust::sort_by_key (BVHBuilder.cu:234) K+4 B in, K+4 B out per pass
-//   k_topology         radix_tree_construction_kernel (:107-201) keys -> Node, parents
-//   k_gather_refit     compute_internal_node_bbox_kernel (:39-98) + the triangle permutation
-//                      + the 96-B traversal nodes (child slots filled bottom-up)
+//   k_tree_blocks      radix_tree_construction_kernel (:107-201), compute_internal_node_bbox_kernel
+//                      (:39-98), the triangle permutation and the 96-B traversal nodes of the
+//                      subtrees inside blocks of 256 leaves
+//   k_tree_top         the same for the nodes across blocks
 //
 // The sort is a least-significant-digit radix sort with 8-bit digits in the
 // onesweep form (one global histogram pass, then one pass per digit in which each
@@ -21,8 +22,8 @@
 // which reproduces thrust's stable sort_by_key order for equal keys. The
 // look-back wait is bounded: after its poll limit (kLookbackPolls, or the
 // caller's CPT_BUILD_LOOKBACK_LIMIT) it records CPT_STATUS_TIMEOUT and proceeds,
-// so no launch can hang; topology and refit then return at once, and the parent
-// walk of the refit is bounded by n - 1 steps.
+// so no launch can hang; the tree's kernels then return at once, and a climb in
+// them widens its leaf range at every step, so it ends.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
@@ -196,53 +197,25 @@ __global__ void __launch_bounds__(kMortonBlock) k_morton(const float* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// Karras radix tree: k_topology (lbvh_common.cuh).
+// Topology, triangle permutation, boxes and traversal records (lbvh_common.cuh): the
+// subtrees inside each block of leaves, then the nodes across blocks.
 // ---------------------------------------------------------------------------
-// Triangle permutation fused with the bottom-up refit. Thread i gathers sorted
-// triangle i (the 40-B reference record), computes its leaf box, then walks up.
-// At each parent it writes its child slot of the parent's 96-B traversal node
-// (the triangle for a leaf, the box for an internal node); the second child to
-// arrive (atomic counter) reads its sibling's box — the box the sibling's thread
-// computed, which for a leaf is the reference's box of the triangle's vertices
-// (BVHBuilder.cu:73-80) — and stores left.unite(right). Below the nodes whose leaf
-// range leaves the block, the counter and the sibling's box live in shared memory
-// (block-scope fences order them); above, the counter increment is a global
-// acquire-release atomic: it publishes this thread's slot and box stores and makes the
-// sibling's visible to the second arriver (the reference's refit has no ordering
-// between them, BVHBuilder.cu:63-86).
-// ---------------------------------------------------------------------------
-#ifndef CPT_REFIT_BLOCK
-#define CPT_REFIT_BLOCK 64
-#endif
-// leaves per block: the nodes below them arrive in shared memory (C5 refit, 16.8 M
-// triangles: 1.67 / 1.70 / 1.77 / 2.01 ms at 64 / 128 / 256 / 512; 2.22 ms all global)
-constexpr int kRefitBlock = CPT_REFIT_BLOCK;
-
-// A climbing thread arrives at node p and learns whether it is the second child to
-// arrive (and may go on). Nodes whose leaf range lies inside this block's leaves have
-// both children completed by threads of this block: they use a shared-memory counter,
-// and the first arriver leaves its box in shared memory for the second. Other nodes
-// use the global counter with acquire-release order, the sibling's box coming from the
-// node-box array (or, for a leaf sibling, its sorted triangle).
-__global__ void __launch_bounds__(kRefitBlock) k_gather_refit(const float* __restrict__ tris_in, const uint32_t* __restrict__ order,
-                                                      uint32_t n, float* __restrict__ tris_out,
-                                                      const uint32_t* __restrict__ children,
-                                                      const uint32_t* __restrict__ parents_leaf,
-                                                      const uint32_t* __restrict__ parents_internal,
-                                                      int* __restrict__ counters, float* __restrict__ nodes,
-                                                      cpt_bbox* __restrict__ node_boxes, uint32_t* __restrict__ status)
+template <typename K>
+__global__ void __launch_bounds__(kTreeBlock, 5) k_tree_blocks(TreeArrays<K> T, TriangleLeaves leaf, TreeList list)
 {
-    __shared__ int s_count[kRefitBlock];
-    __shared__ float s_box[2 * kRefitBlock][6];  // [2 * (p - base) + side]: the first arriver's box
-    const uint32_t base = blockIdx.x * kRefitBlock;
-    s_count[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t i = base + threadIdx.x;
-    if (i >= n) return;
-    if (sort_timed_out(status)) return;  // the order is not a sort: nothing to gather or refit
-    (void)children;
-    gather_refit_leaf(tris_in, order[i], i, n, base, min(n, base + (uint32_t)kRefitBlock), tris_out, parents_leaf,
-                      parents_internal, counters, nodes, node_boxes, status, s_count, s_box);
+    __shared__ TreeSmem sm;
+    if (sort_timed_out(T.status)) return;  // the keys are not sorted: build nothing from them
+    const uint32_t base = blockIdx.x * kTreeBlock;
+    tree_block(sm, T, base, min((uint32_t)kTreeBlock, T.n - base), leaf, list, 0u);
+}
+
+template <typename K>
+__global__ void __launch_bounds__(128) k_tree_top(TreeArrays<K> T, TriangleLeaves leaf, TreeList list)
+{
+    if (sort_timed_out(T.status)) return;
+    const uint32_t m = *list.count;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
+        tree_climb(T, list.first[p], list.last[p], leaf);
 }
 
 // ---------------------------------------------------------------------------
@@ -382,21 +355,21 @@ int build_impl(const cpt_triangle* tris_in, uint32_t n, const float* host_box, c
     // P is even: keys end in bvh->keys, values in vals[(P - 1) & 1].
     const uint32_t* order = s.vals[(P - 1) & 1];
 
-    const uint32_t inner = n - 1;
+    // the list of finished subtrees: the other value buffer and the other key buffer (both
+    // free after the sort, n words and more), counted in a word that k_morton zeroed
+    const TreeArrays<K> T{keys,  n, bvh->children, bvh->parents_leaf, bvh->parents_internal,
+                          static_cast<float*>(bvh->nodes), bvh->node_boxes, s.counters, bvh->status};
+    const TriangleLeaves leaf{tri_src, order, 0u, n, reinterpret_cast<float*>(bvh->tris), bvh->status};
+    const TreeList list{s.vals[P & 1], reinterpret_cast<uint32_t*>(s.keys_alt), s.tile_counters + kTreeListWord};
+    const uint32_t blocks = (n + kTreeBlock - 1) / kTreeBlock;
     {
         CPT_PROF(K_TOPOLOGY, stream);
-        k_topology<K><<<(inner + 255) / 256, 256, 0, stream>>>(keys, n, nullptr, bvh->children, bvh->parents_leaf,
-                                                                bvh->parents_internal, s.counters,
-                                                                static_cast<float4*>(bvh->nodes), bvh->status,
-                                                                inner);
+        k_tree_blocks<K><<<blocks, kTreeBlock, 0, stream>>>(T, leaf, list);
     }
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_GATHER_REFIT, stream);
-        k_gather_refit<<<(n + kRefitBlock - 1) / kRefitBlock, kRefitBlock, 0, stream>>>(tri_src, order, n, reinterpret_cast<float*>(bvh->tris),
-                                                             bvh->children, bvh->parents_leaf, bvh->parents_internal,
-                                                             s.counters, static_cast<float*>(bvh->nodes),
-                                                             bvh->node_boxes, bvh->status);
+        k_tree_top<K><<<tree_top_blocks(blocks, sms), 128, 0, stream>>>(T, leaf, list);
     }
     CPT_LAUNCH_CHECK();
     return CPT_OK;

@@ -15,13 +15,14 @@
 //   k_onesweep          one more stable pass on the scene id: order = (scene, key,
 //                       input position), i.e. each scene's own stable key order
 //   k_batch_keys        each scene's sorted keys, gathered into its output
-//   k_batch_topology    Karras topology of every scene (one thread per internal node)
-//   k_batch_refit       gather + bottom-up refit, blocks never straddling two scenes
+//   k_batch_tree_blocks gather, topology, boxes and records of the subtrees inside blocks of
+//                       leaves, blocks never straddling two scenes
+//   k_batch_tree_top    the nodes across blocks
 //   k_batch_status      the batch's sort / input status copied into every scene's
 //
 // Every scene's outputs are those of cpt_lbvh_build on the same triangles and box,
 // bit for bit: the same key arithmetic, the same stable order (ties by input
-// position), the same topology and refit code (lbvh_common.cuh, lbvh.cu). The scene
+// position), the same tree code (lbvh_common.cuh). The scene
 // table travels by value as a kernel parameter, so a batch build records into a CUDA
 // graph without host-side staging.
 #include <cuda_runtime.h>
@@ -35,8 +36,6 @@
 #include "lbvh_common.cuh"
 
 namespace cpt {
-
-constexpr int kBatchRefitBlock = 64;  // leaves per refit block (as the single build's default)
 
 namespace {
 
@@ -60,7 +59,7 @@ struct BatchTable {
     uint32_t total;                              // N_total
     uint32_t off[CPT_MAX_BATCH_SCENES + 1];      // first global index of each scene
     uint32_t inner_off[CPT_MAX_BATCH_SCENES + 1];  // first global internal node (off - scene)
-    uint32_t block_off[CPT_MAX_BATCH_SCENES + 1];  // first refit block
+    uint32_t block_off[CPT_MAX_BATCH_SCENES + 1];  // first block of leaves
     BatchScene s[CPT_MAX_BATCH_SCENES];
 };
 
@@ -141,41 +140,46 @@ __global__ void __launch_bounds__(kBatchBlock) k_batch_keys(BatchTable bt, const
     }
 }
 
+// Scene sc's arrays; its splits' words start at its first internal node's.
 template <typename K>
-__global__ void __launch_bounds__(256) k_batch_topology(BatchTable bt, int* __restrict__ counters,
-                                                        const uint32_t* __restrict__ batch_status)
+__device__ __forceinline__ TreeArrays<K> batch_tree(const BatchTable& bt, uint32_t sc, int* ends)
 {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t inner_total = bt.total - bt.scenes;
-    if (j >= inner_total) return;
-    if (sort_timed_out(batch_status)) return;
-    const uint32_t sc = segment_of(bt.inner_off, bt.scenes, j);
     const BatchScene& S = bt.s[sc];
-    const int nn = (int)(bt.off[sc + 1] - bt.off[sc]);
-    topology_node(static_cast<const K*>(S.keys), nn, (int)(j - bt.inner_off[sc]), S.children, S.parents_leaf,
-                  S.parents_internal, counters + bt.inner_off[sc], reinterpret_cast<float4*>(S.nodes));
+    return TreeArrays<K>{static_cast<const K*>(S.keys), bt.off[sc + 1] - bt.off[sc], S.children,  S.parents_leaf,
+                         S.parents_internal,            S.nodes,                     S.node_boxes, ends + bt.inner_off[sc],
+                         S.status};
 }
 
-__global__ void __launch_bounds__(kBatchRefitBlock) k_batch_refit(BatchTable bt, const uint32_t* __restrict__ order,
-                                                                  int* __restrict__ counters,
+__device__ __forceinline__ TriangleLeaves batch_leaves(const BatchTable& bt, uint32_t sc, const uint32_t* order)
+{
+    const BatchScene& S = bt.s[sc];
+    return TriangleLeaves{S.tris_in, order + bt.off[sc], bt.off[sc], bt.off[sc + 1] - bt.off[sc], S.tris_out, S.status};
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kTreeBlock, 5) k_batch_tree_blocks(BatchTable bt, const uint32_t* __restrict__ order,
+                                                                  int* __restrict__ ends, TreeList list,
                                                                   const uint32_t* __restrict__ batch_status)
 {
-    __shared__ int s_count[kBatchRefitBlock];
-    __shared__ float s_box[2 * kBatchRefitBlock][6];
-    s_count[threadIdx.x] = 0;
-    __syncthreads();
+    __shared__ TreeSmem sm;
     if (sort_timed_out(batch_status)) return;  // (uniform: set before this launch)
     const uint32_t sc = segment_of(bt.block_off, bt.scenes, blockIdx.x);
-    const BatchScene& S = bt.s[sc];
-    const uint32_t n = bt.off[sc + 1] - bt.off[sc];
-    const uint32_t base = (blockIdx.x - bt.block_off[sc]) * kBatchRefitBlock;
-    const uint32_t i = base + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t v = order[bt.off[sc] + i];
-    const uint32_t src = v >= bt.off[sc] ? v - bt.off[sc] : n;  // n: out of range, reported by the walk
-    gather_refit_leaf(S.tris_in, src, i, n, base, min(n, base + (uint32_t)kBatchRefitBlock), S.tris_out,
-                          S.parents_leaf, S.parents_internal, counters + bt.inner_off[sc], S.nodes, S.node_boxes,
-                          S.status, s_count, s_box);
+    const TreeArrays<K> T = batch_tree<K>(bt, sc, ends);
+    const uint32_t base = (blockIdx.x - bt.block_off[sc]) * kTreeBlock;
+    tree_block(sm, T, base, min((uint32_t)kTreeBlock, T.n - base), batch_leaves(bt, sc, order), list, bt.off[sc]);
+}
+
+template <typename K>
+__global__ void __launch_bounds__(128) k_batch_tree_top(BatchTable bt, const uint32_t* __restrict__ order,
+                                                        int* __restrict__ ends, TreeList list,
+                                                        const uint32_t* __restrict__ batch_status)
+{
+    if (sort_timed_out(batch_status)) return;
+    const uint32_t m = *list.count;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x) {
+        const uint32_t first = list.first[p], sc = segment_of(bt.off, bt.scenes, first);
+        tree_climb(batch_tree<K>(bt, sc, ends), first - bt.off[sc], list.last[p] - bt.off[sc], batch_leaves(bt, sc, order));
+    }
 }
 
 __global__ void k_batch_status(BatchTable bt, const uint32_t* __restrict__ batch_status)
@@ -295,15 +299,18 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
     }
     k_batch_keys<K><<<grid, kBatchBlock, 0, stream>>>(bt, s.keys[0], order);
     CPT_LAUNCH_CHECK();
-    const uint32_t inner_total = bt.total - bt.scenes;
+    // the list of finished subtrees: the scene-id buffers (free after their pass), counted in
+    // a word that k_batch_morton zeroed
+    const TreeList list{s.sid[0], s.sid[1], s.zero + kTreeListWord};
+    const uint32_t blocks = bt.block_off[bt.scenes];
     {
         CPT_PROF(K_TOPOLOGY, stream);
-        k_batch_topology<K><<<(inner_total + 255) / 256, 256, 0, stream>>>(bt, s.counters, s.status);
+        k_batch_tree_blocks<K><<<blocks, kTreeBlock, 0, stream>>>(bt, order, s.counters, list, s.status);
     }
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_GATHER_REFIT, stream);
-        k_batch_refit<<<bt.block_off[bt.scenes], kBatchRefitBlock, 0, stream>>>(bt, order, s.counters, s.status);
+        k_batch_tree_top<K><<<tree_top_blocks(blocks, sms), 128, 0, stream>>>(bt, order, s.counters, list, s.status);
     }
     CPT_LAUNCH_CHECK();
     k_batch_status<<<1, 64, 0, stream>>>(bt, s.status);
@@ -323,7 +330,7 @@ int make_table(const uint32_t* n, uint32_t scenes, BatchTable& bt)
         bt.inner_off[sc] = (uint32_t)(total - sc);
         bt.block_off[sc] = (uint32_t)blocks;
         total += n[sc];
-        blocks += (n[sc] + kBatchRefitBlock - 1) / kBatchRefitBlock;
+        blocks += (n[sc] + kTreeBlock - 1) / kTreeBlock;
         if (total > kMaxTriangles) return CPT_ERR_INVALID_ARGUMENT;  // 30-bit counts in the look-back words
     }
     bt.off[scenes] = (uint32_t)total;

@@ -25,8 +25,9 @@
 //   k_split_emit          pieces, 4 per thread (balanced however the triangles are cut):
 //                         clipped boxes, Morton keys of their centres in the root box,
 //                         digit histograms, zeroed look-back state
-//   k_scan_offsets, k_onesweep x P, k_topology   as the main build, on the device count
-//   k_split_refit         leaf slots + bottom-up boxes into the 96-B traversal nodes
+//   k_scan_offsets, k_onesweep x P   as the main build, on the device count
+//   k_split_tree_blocks, k_split_tree_top   topology, boxes and 96-B traversal nodes, as the main
+//                         build's over leaves that are pieces
 //   k_treelet             (CPT_SPLIT_TREELET) treelet restructuring of the Karras topology
 #include <cuda_runtime.h>
 #include <math.h>
@@ -410,117 +411,82 @@ __global__ void __launch_bounds__(kSplitBlock, 4) k_split_emit(const cpt_triangl
         if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
-__device__ __forceinline__ Box piece_box(const float4* pieces, uint32_t r, bool coherent)
+// Leaves that are pieces: sorted position i holds piece order[i], whose box goes to
+// leaf_boxes; the slot is the whole triangle and its sorted index.
+struct PieceLeaves {
+    const cpt_triangle* tris;
+    const float4* pieces;
+    const uint32_t* order;
+    float4* leaf_boxes;
+    uint32_t n, n_tris;
+    uint32_t* status;
+
+    static __device__ __forceinline__ float lo(float a, float b) { return fminf(a, b); }
+    static __device__ __forceinline__ float hi(float a, float b) { return fmaxf(a, b); }
+    __device__ __forceinline__ void get(uint32_t i, float slot[10], float4& a, float4& b) const
+    {
+        uint32_t src = order[i];
+        if (src >= n) {
+            atomicOr(status, CPT_STATUS_BAD_INDEX);
+            src = n - 1;
+        }
+        a = pieces[2 * (size_t)src];
+        b = pieces[2 * (size_t)src + 1];
+        uint32_t tri = __float_as_uint(a.w);
+        if (tri >= n_tris) {
+            atomicOr(status, CPT_STATUS_BAD_INDEX);
+            tri = n_tris - 1;
+        }
+        const cpt_triangle t = tris[tri];
+        slot[0] = t.v0[0]; slot[1] = t.v0[1]; slot[2] = t.v0[2];
+        slot[3] = __uint_as_float(tri);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            slot[4 + k] = __fsub_rn(t.v1[k], t.v0[k]);
+            slot[7 + k] = __fsub_rn(t.v2[k], t.v0[k]);
+        }
+    }
+    __device__ __forceinline__ void load(uint32_t i, float slot[10], float box[6]) const
+    {
+        float4 a, b;
+        get(i, slot, a, b);
+        box[0] = a.x; box[1] = a.y; box[2] = a.z; box[3] = b.x; box[4] = b.y; box[5] = b.z;
+        leaf_boxes[2 * (size_t)i] = make_float4(a.x, a.y, a.z, 0.f);
+        leaf_boxes[2 * (size_t)i + 1] = make_float4(b.x, b.y, b.z, 0.f);
+    }
+    __device__ __forceinline__ void reload(uint32_t i, float slot[10], float box[6]) const
+    {
+        float4 a, b;
+        get(i, slot, a, b);
+        box[0] = a.x; box[1] = a.y; box[2] = a.z; box[3] = b.x; box[4] = b.y; box[5] = b.z;
+    }
+};
+
+// The split tree over *n_pieces sorted pieces (lbvh_common.cuh); node_cap: the records of
+// `nodes`, those past the tree marked unused.
+template <typename K>
+__global__ void __launch_bounds__(kTreeBlock, 5) k_split_tree_blocks(TreeArrays<K> T, PieceLeaves leaf, TreeList list,
+                                                                  const uint32_t* __restrict__ n_pieces,
+                                                                  uint32_t node_cap)
 {
-    const float4 a = coherent ? __ldcg(pieces + 2 * (size_t)r) : pieces[2 * (size_t)r];
-    const float4 b = coherent ? __ldcg(pieces + 2 * (size_t)r + 1) : pieces[2 * (size_t)r + 1];
-    Box x;
-    x.mn[0] = a.x; x.mn[1] = a.y; x.mn[2] = a.z;
-    x.mx[0] = b.x; x.mx[1] = b.y; x.mx[2] = b.z;
-    return x;
+    __shared__ TreeSmem sm;
+    T.n = leaf.n = *n_pieces;
+    const uint32_t base = blockIdx.x * kTreeBlock, i = base + threadIdx.x;
+    if (i + 1u >= T.n && i < node_cap)
+        reinterpret_cast<float4*>(T.nodes)[6 * (size_t)i + 5] = make_float4(__uint_as_float(kUnusedNode), 0.f, 0.f, 0.f);
+    if (sort_timed_out(T.status) || base >= T.n) return;  // no sorted pieces, or none here (uniform)
+    tree_block(sm, T, base, min((uint32_t)kTreeBlock, T.n - base), leaf, list, 0u);
 }
 
-// Leaf i (sorted piece order[i]): its slot is the whole triangle, its box the
-// piece's; then the bottom-up walk of k_gather_refit with the sibling leaf's box
-// read from the leaf box array.
-// Leaves per block of k_split_refit: nodes whose leaf range (word 22 of the record,
-// written by k_topology) lies inside the block complete in shared memory, as in the
-// LBVH refit; the rest through the global acquire-release counters.
-constexpr int kSplitRefitBlock = 64;
-
-__global__ void __launch_bounds__(kSplitRefitBlock) k_split_refit(const cpt_triangle* __restrict__ tris, const float4* __restrict__ pieces,
-                                                     const uint32_t* __restrict__ order,
-                                                     const uint32_t* __restrict__ n_pieces,
-                                                     const uint32_t* __restrict__ children,
-                                                     const uint32_t* __restrict__ parents_leaf,
-                                                     const uint32_t* __restrict__ parents_internal,
-                                                     int* __restrict__ counters, float* __restrict__ nodes,
-                                                     cpt_bbox* __restrict__ node_boxes, float4* __restrict__ leaf_boxes,
-                                                     uint32_t n_tris, uint32_t* __restrict__ status)
+template <typename K>
+__global__ void __launch_bounds__(128) k_split_tree_top(TreeArrays<K> T, PieceLeaves leaf, TreeList list,
+                                                        const uint32_t* __restrict__ n_pieces)
 {
-    __shared__ int s_count[kSplitRefitBlock];
-    __shared__ float s_box[2 * kSplitRefitBlock][6];  // [2 * (p - base) + side]: the first arriver's box
-    const uint32_t base = blockIdx.x * kSplitRefitBlock;
-    s_count[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t n = *n_pieces;
-    const uint32_t i = base + threadIdx.x;
-    if (i >= n || n < 2) return;
-    if (sort_timed_out(status)) return;  // the pieces are not sorted: no tree to refit
-    const uint32_t block_end = min(n, base + (uint32_t)kSplitRefitBlock);
-    uint32_t src = order[i];
-    if (src >= n) {
-        atomicOr(status, CPT_STATUS_BAD_INDEX);
-        src = n - 1;
-    }
-    Box box = piece_box(pieces, src, false);
-    uint32_t tri = __float_as_uint(pieces[2 * (size_t)src].w);
-    if (tri >= n_tris) {
-        atomicOr(status, CPT_STATUS_BAD_INDEX);
-        tri = n_tris - 1;
-    }
-    leaf_boxes[2 * (size_t)i] = make_float4(box.mn[0], box.mn[1], box.mn[2], 0.f);
-    leaf_boxes[2 * (size_t)i + 1] = make_float4(box.mx[0], box.mx[1], box.mx[2], 0.f);
-    const cpt_triangle t = tris[tri];
-    float slot[10] = {t.v0[0], t.v0[1], t.v0[2], __uint_as_float(tri),
-                      __fsub_rn(t.v1[0], t.v0[0]), __fsub_rn(t.v1[1], t.v0[1]), __fsub_rn(t.v1[2], t.v0[2]),
-                      __fsub_rn(t.v2[0], t.v0[0]), __fsub_rn(t.v2[1], t.v0[1]), __fsub_rn(t.v2[2], t.v0[2])};
-    uint32_t child = i;  // (the leaf box is published by the first arrival's release)
-    uint32_t p = parents_leaf[i];
-    // at most n - 1 nodes on any walk (each node lets one arriver continue)
-    for (uint32_t steps = 0; p != CPT_INVALID_INDEX; ++steps) {
-        if (p >= n - 1 || steps >= n - 1) { atomicOr(status, CPT_STATUS_BAD_INDEX); return; }
-        float* node = nodes + 24 * (size_t)p;
-        const float4 meta = *reinterpret_cast<const float4*>(node + 20);  // Node word, right child, range end
-        const uint32_t word = __float_as_uint(meta.x);
-        const uint32_t left = word >> 2;
-        const int side = left == child ? 0 : 1;
-        const uint32_t j = __float_as_uint(meta.z);
-        const bool local = min(p, j) >= base && max(p, j) < block_end;
-        store_slot(node, side, slot);
-        const uint32_t sib = left + (uint32_t)(1 - side);
-        Box sb;
-        if (local) {
-            const uint32_t k = p - base;
-            float* mine = s_box[2 * k + side];
-#pragma unroll
-            for (int ax = 0; ax < 3; ++ax) { mine[ax] = box.mn[ax]; mine[3 + ax] = box.mx[ax]; }
-            __threadfence_block();
-            const int arrived = atomicAdd(&s_count[k], 1);
-            if (arrived == 0) return;
-            if (arrived != 1) { atomicOr(status, CPT_STATUS_BAD_INDEX); return; }
-            __threadfence_block();
-            const volatile float* other = s_box[2 * k + (1 - side)];
-#pragma unroll
-            for (int ax = 0; ax < 3; ++ax) { sb.mn[ax] = other[ax]; sb.mx[ax] = other[3 + ax]; }
-        } else {
-            const int arrived = arrive_acq_rel(&counters[p]);
-            if (arrived == 0) return;
-            if (arrived != 1) { atomicOr(status, CPT_STATUS_BAD_INDEX); return; }
-            const bool sib_internal = (word >> (1 - side)) & 1u;
-            if (sib_internal) {
-                const float2* q = reinterpret_cast<const float2*>(node_boxes + sib);
-                const float2 x0 = __ldcg(q), x1 = __ldcg(q + 1), x2 = __ldcg(q + 2);
-                sb.mn[0] = x0.x; sb.mn[1] = x0.y; sb.mn[2] = x1.x; sb.mx[0] = x1.y; sb.mx[1] = x2.x; sb.mx[2] = x2.y;
-            } else {
-                sb = piece_box(leaf_boxes, sib, true);
-            }
-        }
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            box.mn[ax] = fminf(box.mn[ax], sb.mn[ax]);
-            box.mx[ax] = fmaxf(box.mx[ax], sb.mx[ax]);
-        }
-        float2* ob = reinterpret_cast<float2*>(node_boxes + p);
-        ob[0] = make_float2(box.mn[0], box.mn[1]);
-        ob[1] = make_float2(box.mn[2], box.mx[0]);
-        ob[2] = make_float2(box.mx[1], box.mx[2]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { slot[k] = box.mn[k]; slot[3 + k] = box.mx[k]; }
-        slot[6] = slot[7] = slot[8] = slot[9] = 0.0f;
-        child = p;
-        p = parents_internal[p];
-    }
+    if (sort_timed_out(T.status)) return;
+    T.n = leaf.n = *n_pieces;
+    const uint32_t m = *list.count;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
+        tree_climb(T, list.first[p], list.last[p], leaf);
 }
 
 // ---------------------------------------------------------------------------
@@ -1094,15 +1060,17 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
         keys = s.keys[P & 1];
     }
     const uint32_t* order = s.vals[(P - 1) & 1];
-    k_topology<K><<<(cap + 255) / 256, 256, 0, stream>>>(keys, 0, s.n_pieces, s.children, s.parents_leaf,
-                                                          s.parents_internal, s.counters, static_cast<float4*>(nodes),
-                                                          bvh->status, cap - 1);
+    // the list of finished subtrees: the other value and key buffers, free after the sort,
+    // counted in a word that k_split_emit zeroed
+    const TreeArrays<K> T{keys,        0u, s.children, s.parents_leaf, s.parents_internal, static_cast<float*>(nodes),
+                          s.node_boxes, s.counters, bvh->status};
+    const PieceLeaves leaf{bvh->tris, s.pieces, order, s.leaf_boxes, 0u, n, bvh->status};
+    const TreeList list{s.vals[P & 1], reinterpret_cast<uint32_t*>(keys == s.keys[0] ? s.keys[1] : s.keys[0]),
+                        s.zero + kTreeListWord};
+    const uint32_t blocks = (cap + kTreeBlock - 1) / kTreeBlock;
+    k_split_tree_blocks<K><<<blocks, kTreeBlock, 0, stream>>>(T, leaf, list, s.n_pieces, cap - 1);
     CPT_LAUNCH_CHECK();
-    k_split_refit<<<(cap + kSplitRefitBlock - 1) / kSplitRefitBlock, kSplitRefitBlock, 0, stream>>>(
-        bvh->tris, s.pieces, order, s.n_pieces, s.children,
-                                                          s.parents_leaf, s.parents_internal, s.counters,
-                                                          static_cast<float*>(nodes), s.node_boxes, s.leaf_boxes, n,
-                                                          bvh->status);
+    k_split_tree_top<K><<<tree_top_blocks(blocks, sm_count()), 128, 0, stream>>>(T, leaf, list, s.n_pieces);
     CPT_LAUNCH_CHECK();
     if (treelet) {
         for (int round = 0; round < kTreeletRounds; ++round) {
