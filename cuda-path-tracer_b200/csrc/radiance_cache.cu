@@ -54,12 +54,20 @@ constexpr size_t kTrainSmem = sizeof(bf16) * ((size_t)kWSmem + (size_t)kTrainRow
                                               (size_t)kTrainRows * kZS);
 constexpr size_t kInferSmem = sizeof(bf16) * ((size_t)kWSmem + (size_t)kInferWarps * 16 * kXS);
 
-__device__ __forceinline__ void box_params(const float* box, float (&bmin)[3], float (&binv)[3])
+// The box that normalises positions: a caller's by value, or a scene's on the device.
+struct RcBox {
+    float v[6];
+    const float* dev;  // nullable
+};
+inline RcBox host_box(const float* b) { return {{b[0], b[1], b[2], b[3], b[4], b[5]}, nullptr}; }
+inline RcBox device_box(const float* b) { return {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, b}; }
+
+__device__ __forceinline__ void box_params(const RcBox& box, float (&bmin)[3], float (&binv)[3])
 {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        bmin[a] = box[a];
-        const float ext = box[3 + a] - box[a];
+        bmin[a] = box.dev ? box.dev[a] : box.v[a];
+        const float ext = (box.dev ? box.dev[3 + a] : box.v[3 + a]) - bmin[a];
         binv[a] = ext > 0.f ? 1.0f / ext : 0.f;
     }
 }
@@ -73,16 +81,20 @@ __device__ __forceinline__ void batch_range(const uint32_t* count_dev, uint32_t 
 }
 
 // ---------------------------------------------------------------------------
-// inference
+// inference: issue slots (the encoding's 36 sines and cosines) and the tensor pipe take turns, 56 %
+// and 47 % busy at 24 warps per SM. A million samples: 155 us; 136 with the encoding balanced over
+// the two lanes of a row and the next rows prefetched. 32 rows per warp (each weight fragment
+// loaded once for both tiles, shared-memory wavefronts 61 -> 36 %) is no faster: 136, and 24.2
+// against 25.3 for 100,000 but 14.7 against 12.1 for 1,000.
 
 // kRecords = false: `in` holds samples (4 float4 each), out[i] = (rgb, 0).
 // kRecords = true: `in` holds render records (5 float4 each: position | path id,
 // direction | W.x, normal | W.y, albedo | W.z, R1); the path's radiance in `out`
 // (the wavefront state, 2 float4 per path) gains W * max(prediction, 0).
 template <bool kRecords>
-__global__ void __launch_bounds__(kInferBlock) k_rc_infer(const bf16* __restrict__ w, const float4* __restrict__ in,
+__global__ void __launch_bounds__(kInferBlock, 3) k_rc_infer(const bf16* __restrict__ w, const float4* __restrict__ in,
                                                           const uint32_t* __restrict__ count_dev, uint32_t count_host,
-                                                          const float* __restrict__ box, float4* __restrict__ out)
+                                                          RcBox box, float4* __restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* ws = reinterpret_cast<bf16*>(smem_raw);
@@ -98,6 +110,10 @@ __global__ void __launch_bounds__(kInferBlock) k_rc_infer(const bf16* __restrict
     for (uint32_t t = blockIdx.x * kInferWarps + warp; t < tiles; t += gridDim.x * kInferWarps) {
         const uint32_t base = t * 16;
         const int r = lane & 15;
+        {  // the next tile's rows into L2
+            const uint64_t next = (uint64_t)base + (uint64_t)gridDim.x * kInferWarps * 16 + (uint32_t)r;
+            if (next < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(in + (size_t)kF4 * next));
+        }
         const uint32_t gi = base + r;
         const bool valid = gi < n;
         float4 f[4];
@@ -214,8 +230,7 @@ __global__ void __launch_bounds__(kTrainBlock, 1) k_rc_train(const bf16* __restr
                                                              const float4* __restrict__ samples,
                                                              const uint32_t* __restrict__ count_dev,
                                                              uint32_t count_host, uint32_t step, uint32_t steps,
-                                                             const float* __restrict__ box,
-                                                             float* __restrict__ partials, float* __restrict__ loss)
+                                                             RcBox box, float* __restrict__ partials, float* __restrict__ loss)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* ws = reinterpret_cast<bf16*>(smem_raw);
@@ -318,18 +333,38 @@ struct AdamArgs {
     const uint32_t* count_dev;
 };
 
-__global__ void __launch_bounds__(256) k_rc_adam(const float* __restrict__ partials, float* __restrict__ master,
+// A block's 128 parameters of up to 148 blocks' partial gradients at once in shared memory (one
+// asynchronous copy each thread and row quarter, all under way together), then added in block
+// order: a thread that loads its own column keeps a few loads in flight and took 11 to 13 us a
+// step for these 11.5 MB; now 9.2.
+constexpr int kAdamBlock = 128, kAdamRows = 148;
+constexpr size_t kAdamSmem = sizeof(float) * kAdamRows * kAdamBlock;
+static_assert(kParams % kAdamBlock == 0, "whole blocks of parameters");
+__global__ void __launch_bounds__(kAdamBlock) k_rc_adam(const float* __restrict__ partials, float* __restrict__ master,
                                                  float* __restrict__ m1, float* __restrict__ m2,
                                                  float* __restrict__ ema, bf16* __restrict__ w_train,
                                                  bf16* __restrict__ w_infer, AdamArgs a)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kParams) return;
+    extern __shared__ __align__(16) float s_part[];
+    const int i = blockIdx.x * kAdamBlock + threadIdx.x;
     uint32_t lo, hi;
     batch_range(a.count_dev, a.count_host, a.step, a.steps, lo, hi);
     if (hi == lo) return;  // empty batch: no step
     float g = 0.f;
-    for (int p = 0; p < a.parts; ++p) g += partials[(size_t)p * kParams + i];
+    for (int p0 = 0; p0 < a.parts; p0 += kAdamRows) {
+        const int rows = min(kAdamRows, a.parts - p0);
+        const int first = blockIdx.x * kAdamBlock;
+        for (int q = threadIdx.x; q < rows * (kAdamBlock / 4); q += kAdamBlock) {
+            const int r = q / (kAdamBlock / 4), c = 4 * (q % (kAdamBlock / 4));
+            const uint32_t dst = smem_addr(s_part + r * kAdamBlock + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst),
+                         "l"(partials + (size_t)(p0 + r) * kParams + first + c));
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        for (int r = 0; r < rows; ++r) g += s_part[r * kAdamBlock + threadIdx.x];
+        __syncthreads();
+    }
     const float m = a.beta1 * m1[i] + (1.0f - a.beta1) * g;
     const float v = a.beta2 * m2[i] + (1.0f - a.beta2) * g * g;
     m1[i] = m;
@@ -415,7 +450,6 @@ struct cpt_rc {
     float* partials = nullptr;
     int parts = 0;
     float* loss = nullptr;      // [2] per cpt_rc_train call
-    float* box = nullptr;       // [6] normalisation box for host-supplied boxes
     float4* samples = nullptr;  // training samples of the current frame
     uint32_t* sample_count = nullptr;
     uint32_t sample_cap = 0;
@@ -445,6 +479,7 @@ int set_attributes()
     CPT_CUDA_TRY(cudaFuncSetAttribute(k_rc_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
     CPT_CUDA_TRY(cudaFuncSetAttribute(k_rc_infer<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
     CPT_CUDA_TRY(cudaFuncSetAttribute(k_rc_infer<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_rc_adam, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdamSmem));
     g_attr_done[dev] = true;
     return CPT_OK;
 }
@@ -462,7 +497,7 @@ int infer_grid()
 
 // One training batch (step `step` of `steps` over the sample set) + Adam.
 int train_batch(cpt_rc* rc, const float4* samples, const uint32_t* count_dev, uint32_t count_host, uint32_t step,
-                uint32_t steps, const float* box, float* loss, cudaStream_t stream)
+                uint32_t steps, const RcBox& box, float* loss, cudaStream_t stream)
 {
     {
         CPT_PROF(K_RC_TRAIN, stream);
@@ -487,7 +522,7 @@ int train_batch(cpt_rc* rc, const float4* samples, const uint32_t* count_dev, ui
     a.steps = steps;
     {
         CPT_PROF(K_RC_ADAM, stream);
-        k_rc_adam<<<(kParams + 255) / 256, 256, 0, stream>>>(rc->partials, rc->master, rc->m1, rc->m2, rc->ema,
+        k_rc_adam<<<kParams / kAdamBlock, kAdamBlock, kAdamSmem, stream>>>(rc->partials, rc->master, rc->m1, rc->m2, rc->ema,
                                                              rc->w_train, rc->w_infer, a);
     }
     CPT_LAUNCH_CHECK();
@@ -496,7 +531,7 @@ int train_batch(cpt_rc* rc, const float4* samples, const uint32_t* count_dev, ui
 
 struct Ctx {
     cpt_rc* rc;
-    const float* box;
+    RcBox box;
     bool training;    // a training-only pass: every record is a training record
     bool own_paths;   // an image pass with training paths among its own paths
 };
@@ -585,7 +620,6 @@ extern "C" int cpt_rc_create(cpt_rc** out, const cpt_rc_params* params, cudaStre
     c.take<bf16>(kParams);
     c.take<float>((size_t)rc->parts * kParams);
     c.take<float>(2);
-    c.take<float>(6);
     c.take<float4>(4ull * rc->sample_cap);
     c.take<uint32_t>(1);
     rc->train_cap = p.train_samples;
@@ -604,7 +638,6 @@ extern "C" int cpt_rc_create(cpt_rc** out, const cpt_rc_params* params, cudaStre
     rc->w_infer = d.take<bf16>(kParams);
     rc->partials = d.take<float>((size_t)rc->parts * kParams);
     rc->loss = d.take<float>(2);
-    rc->box = d.take<float>(6);
     rc->samples = d.take<float4>(4ull * rc->sample_cap);
     rc->sample_count = d.take<uint32_t>(1);
     rc->train_records = d.take<float4>(5ull * rc->train_cap);
@@ -663,15 +696,14 @@ extern "C" int cpt_rc_infer(cpt_rc* rc, const float* samples, uint32_t n, const 
     CPT_RANGE("cpt_rc_infer");
     if (!rc || !box || (n && (!samples || !out))) return CPT_ERR_INVALID_ARGUMENT;
     if (!n) return CPT_OK;
-    CPT_CUDA_TRY(cudaMemcpyAsync(rc->box, box, 6 * sizeof(float), cudaMemcpyHostToDevice, stream));
     {
         CPT_PROF(K_RC_INFER, stream);
         const int grid = std::min<int>(infer_grid(), (int)((n + 16 * kInferWarps - 1) / (16 * kInferWarps)));
         k_rc_infer<false><<<grid, kInferBlock, kInferSmem, stream>>>(
-            rc->w_infer, reinterpret_cast<const float4*>(samples), nullptr, n, rc->box, reinterpret_cast<float4*>(out));
+            rc->w_infer, reinterpret_cast<const float4*>(samples), nullptr, n, host_box(box), reinterpret_cast<float4*>(out));
     }
     CPT_LAUNCH_CHECK();
-    CPT_CUDA_TRY(cudaStreamSynchronize(stream));  // the host box may go away
+    CPT_CUDA_TRY(cudaStreamSynchronize(stream));
     return CPT_OK;
 }
 
@@ -680,10 +712,9 @@ extern "C" int cpt_rc_train(cpt_rc* rc, const float* samples, uint32_t n, const 
 {
     CPT_RANGE("cpt_rc_train");
     if (!rc || !box || !samples || n == 0 || steps == 0) return CPT_ERR_INVALID_ARGUMENT;
-    CPT_CUDA_TRY(cudaMemcpyAsync(rc->box, box, 6 * sizeof(float), cudaMemcpyHostToDevice, stream));
     CPT_CUDA_TRY(cudaMemsetAsync(rc->loss, 0, 2 * sizeof(float), stream));
     for (uint32_t s = 0; s < steps; ++s) {
-        const int r = train_batch(rc, reinterpret_cast<const float4*>(samples), nullptr, n, s, steps, rc->box, rc->loss,
+        const int r = train_batch(rc, reinterpret_cast<const float4*>(samples), nullptr, n, s, steps, host_box(box), rc->loss,
                                   stream);
         if (r) return r;
     }
@@ -741,7 +772,7 @@ int rc_frame(cpt_rc* rc, const cpt_view* views, uint32_t n_views, const cpt_rend
     const size_t rec_r = render_hook_layout(views, n_views, params, nullptr, &cap_r);
     const size_t render_part = need - std::max(rec_t, rec_r);
     float4* records = reinterpret_cast<float4*>(static_cast<char*>(scratch) + render_part);
-    const float* box = reinterpret_cast<const float*>(views[0].bvh->node_boxes);
+    const RcBox box = device_box(reinterpret_cast<const float*>(views[0].bvh->node_boxes));
     const uint32_t steps = rc->params.train_steps;
     if (!image) {
         // training only (cpt_rc_update): full-depth paths over reduced copies of the views,

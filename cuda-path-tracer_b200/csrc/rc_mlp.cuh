@@ -159,11 +159,14 @@ __device__ __forceinline__ void sh16(float x, float y, float z, float (&o)[16])
 }
 
 // Writes half of one encoded row (BF16 pairs as 32-bit stores):
-//   half 0: position axes 0, 1 -> columns 0..47
-//   half 1: position axis 2 -> 48..71, SH(direction) -> 72..87, normal -> 88..90,
-//           albedo -> 91..93, constant 1 -> 94, 0 -> 95.
-// Position p = (x - box_min) / (box_max - box_min); column 24a + 2k holds
-// sin(pi 2^k p_a) and 24a + 2k + 1 its cosine. valid = false writes zeros.
+//   columns 0..71: position p = (x - box_min) / (box_max - box_min), 24a + 2k holds
+//   sin(pi 2^k p_a) and 24a + 2k + 1 its cosine; 72..87 SH(direction), 88..90 normal, 91..93
+//   albedo, 94 a constant 1, 95 a 0.
+// half 0: axis 0 and the lower six frequencies of axis 1; half 1: axis 2, the upper six of
+// axis 1 and the rest. Both halves run the same 18 sines and cosines together (with an axis
+// and a half more for half 0 than for half 1 a warp ran 24 passes of them, the other half's
+// lanes idle), and 2^k p is a product (exact, as ldexpf(p, k), which takes ten instructions).
+// valid = false writes zeros.
 __device__ __forceinline__ void encode_half(const float4* f, bool valid, const float* bmin, const float* binv, int half,
                                             __nv_bfloat16* row)
 {
@@ -173,16 +176,22 @@ __device__ __forceinline__ void encode_half(const float4* f, bool valid, const f
         for (int k = 0; k < 24; ++k) out[half * 24 + k] = 0u;
         return;
     }
-    const float pos[3] = {f[0].x, f[0].y, f[0].z};
-    const int a0 = half == 0 ? 0 : 2, a1 = half == 0 ? 2 : 3;
-    for (int a = a0; a < a1; ++a) {
-        const float p = (pos[a] - bmin[a]) * binv[a];
+    const int a = half ? 2 : 0;
+    const float pa = ((half ? f[0].z : f[0].x) - (half ? bmin[2] : bmin[0])) * (half ? binv[2] : binv[0]);
+    const float pb = __fmul_rn((f[0].y - bmin[1]) * binv[1], half ? 64.0f : 1.0f);
+    uint32_t* oa = out + 12 * a;
+    uint32_t* ob = out + 12 + (half ? 6 : 0);
 #pragma unroll
-        for (int k = 0; k < kFreqs; ++k) {
-            float s, c;
-            sincospif(ldexpf(p, k), &s, &c);
-            out[12 * a + k] = pack_bf16(s, c);
-        }
+    for (int k = 0; k < kFreqs; ++k) {
+        float s, c;
+        sincospif(__fmul_rn(pa, (float)(1 << k)), &s, &c);
+        oa[k] = pack_bf16(s, c);
+    }
+#pragma unroll
+    for (int k = 0; k < kFreqs / 2; ++k) {
+        float s, c;
+        sincospif(__fmul_rn(pb, (float)(1 << k)), &s, &c);
+        ob[k] = pack_bf16(s, c);
     }
     if (half == 1) {
         float sh[16];
