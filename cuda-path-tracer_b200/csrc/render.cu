@@ -270,6 +270,11 @@ __global__ void __launch_bounds__(kGenBlock) k_generate(Wave wv, Views vs, float
     }
 }
 
+// A refill of rays of several views loads each ray's tree as well, so it waits for more lanes
+// than one of a single scene (kWideRefillLanes; twelve scenes of 5,000 to 50,000 triangles:
+// 10.2 ms a frame at 31, 9.9 at 28, 10.1 at 24).
+constexpr int kViewsRefillLanes = 28;
+
 // kOneView: every ray traverses view 0's BVH (a single scene, e.g. several cameras of
 // it); the node array is then a kernel-wide constant instead of a per-ray value.
 #ifndef CPT_EXTEND_MIN_BLOCKS
@@ -305,8 +310,7 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(
         };
         persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false, !kStats>(
             wide_of, queue, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, order,
-            WideHits{hits},
-            refill);
+            WideHits{hits}, refill ? refill : kOneView ? (uint32_t)kWideRefillLanes : (uint32_t)kViewsRefillLanes);
         if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
         if (kStats && ray_counts) {
             warp_count_u64(ray_counts + 3, nn);

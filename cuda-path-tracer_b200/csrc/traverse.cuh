@@ -317,9 +317,12 @@ __device__ __forceinline__ Hit traverse(const float4* __restrict__ nodes, f3 o, 
 // taken, visits the next node of the node group (the rest of the group goes on the
 // stack; the node's triangle group queues behind), or pops a group. The triangle test
 // is tri_test on the binary leaf slot's words, so a hit's t, u, v are unchanged.
-// stack entries (2 words) per thread in shared memory (8, 12 and 16 run alike; with the words
-// that share a launch's last rays, 8 blocks of 128 threads stay within a 164 KB split)
-constexpr int kWideSmemStack = 15;
+// stack entries (2 words) per thread in shared memory: with 11, and the words that share a
+// launch's last rays, 8 blocks of 128 threads fit a 132 KB split, and the L1 cache is 32 KB
+// larger than with 12 to 15 (C1 805 -> 782 us, a viewer's frame 3.51 -> 3.43 ms, C2 93.6 -> 92.8);
+// with 8, 6 or 3 entries (100, 100 and 64 KB) those in local memory cost what the cache gives or
+// more (one million rays 2.91 -> 2.96, 3.26 and 3.59 ms)
+constexpr int kWideSmemStack = 11;
 constexpr float kWideGrow = 1.0f + 1.0f / 262144.0f;  // relative slack of a wide child's box test
 // Records a leaf slot holds at most: binary subtrees of up to this many leaves become one
 // leaf slot of their parent wide node instead of a wide node of their own; a wide tree
