@@ -204,6 +204,8 @@ template <typename K>
 __global__ void __launch_bounds__(kTreeBlock, 5) k_tree_blocks(TreeArrays<K> T, TriangleLeaves leaf, TreeList list)
 {
     __shared__ TreeSmem sm;
+    wait_for_previous();
+    let_next_start();
     if (sort_timed_out(T.status)) return;  // the keys are not sorted: build nothing from them
     const uint32_t base = blockIdx.x * kTreeBlock;
     tree_block(sm, T, base, min((uint32_t)kTreeBlock, T.n - base), leaf, list, 0u);
@@ -212,6 +214,8 @@ __global__ void __launch_bounds__(kTreeBlock, 5) k_tree_blocks(TreeArrays<K> T, 
 template <typename K>
 __global__ void __launch_bounds__(128) k_tree_top(TreeArrays<K> T, TriangleLeaves leaf, TreeList list)
 {
+    wait_for_previous();
+    let_next_start();
     if (sort_timed_out(T.status)) return;
     const uint32_t m = *list.count;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
@@ -347,7 +351,7 @@ int build_impl(const cpt_triangle* tris_in, uint32_t n, const float* host_box, c
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_SCAN, stream);
-        k_scan_offsets<<<P, kRadix, 0, stream>>>(s.hist, s.offsets);
+        launch_early(k_scan_offsets, P, kRadix, 0, stream, s.hist, s.offsets);
     }
     CPT_LAUNCH_CHECK();
 
@@ -364,12 +368,12 @@ int build_impl(const cpt_triangle* tris_in, uint32_t n, const float* host_box, c
     const uint32_t blocks = (n + kTreeBlock - 1) / kTreeBlock;
     {
         CPT_PROF(K_TOPOLOGY, stream);
-        k_tree_blocks<K><<<blocks, kTreeBlock, 0, stream>>>(T, leaf, list);
+        launch_early(k_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list);
     }
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_GATHER_REFIT, stream);
-        k_tree_top<K><<<tree_top_blocks(blocks, sms), 128, 0, stream>>>(T, leaf, list);
+        launch_early(k_tree_top<K>, tree_top_blocks(blocks, sms), 128, 0, stream, T, leaf, list);
     }
     CPT_LAUNCH_CHECK();
     return CPT_OK;

@@ -162,6 +162,8 @@ __global__ void __launch_bounds__(kTreeBlock, 5) k_batch_tree_blocks(BatchTable 
                                                                   const uint32_t* __restrict__ batch_status)
 {
     __shared__ TreeSmem sm;
+    wait_for_previous();
+    let_next_start();
     if (sort_timed_out(batch_status)) return;  // (uniform: set before this launch)
     const uint32_t sc = segment_of(bt.block_off, bt.scenes, blockIdx.x);
     const TreeArrays<K> T = batch_tree<K>(bt, sc, ends);
@@ -174,6 +176,8 @@ __global__ void __launch_bounds__(128) k_batch_tree_top(BatchTable bt, const uin
                                                         int* __restrict__ ends, TreeList list,
                                                         const uint32_t* __restrict__ batch_status)
 {
+    wait_for_previous();
+    let_next_start();
     if (sort_timed_out(batch_status)) return;
     const uint32_t m = *list.count;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x) {
@@ -252,7 +256,7 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_SCAN, stream);
-        k_scan_offsets<<<P + 1, kRadix, 0, stream>>>(s.hist, s.offsets);
+        launch_early(k_scan_offsets, P + 1, kRadix, 0, stream, s.hist, s.offsets);
     }
     CPT_LAUNCH_CHECK();
     const uint32_t tiles = sort_tiles(bt.total);
@@ -305,12 +309,13 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
     const uint32_t blocks = bt.block_off[bt.scenes];
     {
         CPT_PROF(K_TOPOLOGY, stream);
-        k_batch_tree_blocks<K><<<blocks, kTreeBlock, 0, stream>>>(bt, order, s.counters, list, s.status);
+        launch_early(k_batch_tree_blocks<K>, blocks, kTreeBlock, 0, stream, bt, order, s.counters, list, s.status);
     }
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_GATHER_REFIT, stream);
-        k_batch_tree_top<K><<<tree_top_blocks(blocks, sms), 128, 0, stream>>>(bt, order, s.counters, list, s.status);
+        launch_early(k_batch_tree_top<K>, tree_top_blocks(blocks, sms), 128, 0, stream, bt, order, s.counters, list,
+                     s.status);
     }
     CPT_LAUNCH_CHECK();
     k_batch_status<<<1, 64, 0, stream>>>(bt, s.status);
