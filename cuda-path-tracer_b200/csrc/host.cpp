@@ -19,6 +19,8 @@ namespace cpt {
 std::atomic<unsigned long long> g_launches{0};
 std::atomic<bool> g_profiling{false};
 
+// (k_topology counts the tree kernels' blocks, k_gather_refit the nodes across blocks: the names
+// that callers look up)
 const char* const kKernelNames[K_KERNEL_COUNT] = {
     "k_bounds", "k_morton", "k_scan_offsets", "k_onesweep", "k_topology", "k_gather_refit", "k_trace",
     "k_generate", "k_extend", "k_shade", "k_wave_counts", "k_accumulate", "k_resolve", "k_ray_sort",

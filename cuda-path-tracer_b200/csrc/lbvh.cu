@@ -1,5 +1,5 @@
 // LBVH construction for sm_100a: Morton codes, onesweep radix sort, Karras
-// topology, atomic bottom-up refit.
+// topology and boxes in blocks of leaves, then across them.
 //
 // Replaces CUDA::BVHBuilder::build (source/application/cuda/BVHBuilder.cu:207-269)
 // and its four thrust passes. Outputs are the reference's arrays, bit for bit,

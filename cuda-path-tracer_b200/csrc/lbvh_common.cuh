@@ -1,6 +1,6 @@
 // Pieces of the LBVH build shared by the reference-format build (lbvh.cu) and
-// the split traversal BVH (split.cu): key traits and Morton helpers, the Karras
-// topology kernel, box helpers and the 40-B traversal child slot.
+// the split traversal BVH (split.cu): key traits and Morton helpers, box helpers, the 40-B
+// traversal child slot, and the radix tree with its boxes and records.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -60,6 +60,6 @@ extern "C" int cpt_lbvh_build_static(const cpt_triangle* tris_in, uint32_t n, co
     const int rc = scratch_address(&scratch);
     if (rc != CPT_OK) return rc;
     // Same build as cpt_lbvh_build; everything the build needs at zero it zeroes
-    // itself on the stream (histograms, look-back words, refit counters, status).
+    // itself on the stream (histograms, look-back words, the tree kernels' list, status).
     return cpt_lbvh_build(tris_in, n, enclosing_box, morton_bits, bvh, scratch, kStaticScratchBytes, flags, stream);
 }

@@ -496,9 +496,9 @@ __global__ void __launch_bounds__(128) k_split_tree_top(TreeArrays<K> T, PieceLe
 // ---------------------------------------------------------------------------
 // Treelet restructuring (CPT_SPLIT_TREELET; Karras and Aila, "Fast Parallel
 // Construction of High-Quality Bounding Volume Hierarchies", HPG 2013), applied to
-// the split tree after its refit. The cost of a tree is the sum of the surface
+// the split tree after its boxes. The cost of a tree is the sum of the surface
 // areas of its internal nodes (the surface-area heuristic with the leaves fixed:
-// every piece stays one leaf). A bottom-up walk with the refit's arrival counters
+// every piece stays one leaf). A bottom-up walk with arrival counters
 // reaches a node once both its subtrees are final; where the node has at least
 // gamma leaves, its warp forms a treelet — the node's two children, then, up to 7
 // leaves, the internal treelet leaf of largest area replaced by its two children —

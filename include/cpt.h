@@ -118,8 +118,8 @@ int cpt_lbvh_build(const cpt_triangle* tris_in, uint32_t n, const float* enclosi
 
 /* Batched LBVH build: the LBVHs of `scenes` triangle soups in one fixed sequence of
  * launches, each launch covering every scene (one Morton launch, one stable radix
- * sort over all scenes — the key digits, then a scene-id digit —, one topology launch,
- * one refit launch). Replaces `scenes` calls of CUDA::BVHBuilder::build
+ * sort over all scenes — the key digits, then a scene-id digit —, two launches for the trees).
+ * Replaces `scenes` calls of CUDA::BVHBuilder::build
  * (source/application/cuda/BVHBuilder.cu:207-269), one per scene; every scene's
  * outputs are bit-identical to cpt_lbvh_build's on the same triangles and box.
  * Host arrays of `scenes` entries: tris_in[s] (device triangles; may equal
@@ -168,7 +168,7 @@ int cpt_lbvh_build_static(const cpt_triangle* tris_in, uint32_t n, const float* 
  * axis, each piece keeping the box of the triangle clipped to its slab (widened by
  * 2^-20 of the coordinates so rounding cannot lose a hit); the pieces get their
  * own LBVH (Morton keys of the piece box centres in the root box, the same sort,
- * topology and refit kernels). The extra pieces are shared out in proportion to
+ * tree kernels). The extra pieces are shared out in proportion to
  * sqrt(box area - 2 x triangle area), at most extra_ratio x n of them. Leaves hold
  * the whole triangle and its sorted index, so tracing reports the same triangles
  * (t, u, v and index) as over `nodes`, except that of two triangles hit at exactly
