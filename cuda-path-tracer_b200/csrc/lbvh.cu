@@ -351,7 +351,7 @@ int build_impl(const cpt_triangle* tris_in, uint32_t n, const float* host_box, c
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_SCAN, stream);
-        launch_early(k_scan_offsets, P, kRadix, 0, stream, s.hist, s.offsets);
+        launch_early(start_early(n), k_scan_offsets, P, kRadix, 0, stream, s.hist, s.offsets);
     }
     CPT_LAUNCH_CHECK();
 
@@ -368,12 +368,12 @@ int build_impl(const cpt_triangle* tris_in, uint32_t n, const float* host_box, c
     const uint32_t blocks = (n + kTreeBlock - 1) / kTreeBlock;
     {
         CPT_PROF(K_TOPOLOGY, stream);
-        launch_early(k_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list);
+        launch_early(start_early(n), k_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list);
     }
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_GATHER_REFIT, stream);
-        launch_early(k_tree_top<K>, tree_top_blocks(blocks, sms), 128, 0, stream, T, leaf, list);
+        launch_early(start_early(n), k_tree_top<K>, tree_top_blocks(blocks, sms), 128, 0, stream, T, leaf, list);
     }
     CPT_LAUNCH_CHECK();
     return CPT_OK;

@@ -256,7 +256,7 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_SCAN, stream);
-        launch_early(k_scan_offsets, P + 1, kRadix, 0, stream, s.hist, s.offsets);
+        launch_early(start_early(bt.total), k_scan_offsets, P + 1, kRadix, 0, stream, s.hist, s.offsets);
     }
     CPT_LAUNCH_CHECK();
     const uint32_t tiles = sort_tiles(bt.total);
@@ -309,13 +309,14 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
     const uint32_t blocks = bt.block_off[bt.scenes];
     {
         CPT_PROF(K_TOPOLOGY, stream);
-        launch_early(k_batch_tree_blocks<K>, blocks, kTreeBlock, 0, stream, bt, order, s.counters, list, s.status);
+        launch_early(start_early(bt.total), k_batch_tree_blocks<K>, blocks, kTreeBlock, 0, stream, bt, order,
+                     s.counters, list, s.status);
     }
     CPT_LAUNCH_CHECK();
     {
         CPT_PROF(K_GATHER_REFIT, stream);
-        launch_early(k_batch_tree_top<K>, tree_top_blocks(blocks, sms), 128, 0, stream, bt, order, s.counters, list,
-                     s.status);
+        launch_early(start_early(bt.total), k_batch_tree_top<K>, tree_top_blocks(blocks, sms), 128, 0, stream, bt,
+                     order, s.counters, list, s.status);
     }
     CPT_LAUNCH_CHECK();
     k_batch_status<<<1, 64, 0, stream>>>(bt, s.status);

@@ -51,18 +51,25 @@ struct SortWait {
     uint32_t withhold_tile0 = 0;
 };
 
-// A kernel launched by launch_early may start while the one before it on the stream drains: its
-// blocks are set up as soon as every block of that one has called let_next_start (or ended) and
-// wait in wait_for_previous until it has completed and its writes are visible. The kernel calls
-// wait_for_previous before it touches memory. (A kernel whose blocks wait on one another lets
-// the next start when all of them are running, so those cannot take their place.) The launches
-// of a sort and of a tree are short and follow on one another: 65,538 triangles, eight launches,
-// 98.8 -> 92.2 us a build.
+// A kernel launched by launch_early with `early` may start while the one before it on the stream
+// drains: its blocks are set up as soon as every block of that one has called let_next_start (or
+// ended) and wait in wait_for_previous until it has completed and its writes are visible. The
+// kernel calls wait_for_previous before it touches memory. (A kernel whose blocks wait on one
+// another lets the next start when all of them are running, so those cannot take their place.)
+// The launches of a sort and of a tree follow on one another, and are short for small inputs:
+// 65,538 triangles, eight launches, 98.8 -> 92.2 us a build. Large ones gain nothing to speak of
+// (5.24 M: 1,223 -> 1,214 us), and their waiting blocks take room from other streams: a frame
+// traced while the next scene is built, 129 -> 140 ms. So launches of few elements alone start
+// early (start_early).
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Elements up to which a sort's and a tree's launches start early.
+inline bool start_early(uint64_t n) { return n <= kSortSmall; }
+
 template <typename... P, typename... A>
-inline void launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, const A&... args)
+inline void launch_early(bool early, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream,
+                         const A&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -73,7 +80,7 @@ inline void launch_early(void (*kernel)(P...), int grid, int block, size_t smem,
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // (CPT_LAUNCH_CHECK reads the error)
 }
 
@@ -379,20 +386,23 @@ inline int onesweep_sort64_halves_t(const uint64_t* keys_in, uint64_t* keys_out,
         const uint32_t* off = offsets + p * kRadix;
         SortWait w = wait;
         if (p) w.withhold_tile0 = 0;  // (the test hook stalls the first pass only)
+        const bool early = start_early(cap);
         auto launch = [&]() {
             if (p == 0)
-                launch_early(k_onesweep_halves<uint32_t, kSrcLow64, kItems>, tiles, kSortBlock, smem32, stream,
-                    nullptr, nullptr, keys_in, half[0], vout, n, n_ptr, 0, off, lb, tile_counters + p, status, w);
+                launch_early(early, k_onesweep_halves<uint32_t, kSrcLow64, kItems>, tiles, kSortBlock, smem32, stream,
+                             nullptr, nullptr, keys_in, half[0], vout, n, n_ptr, 0, off, lb, tile_counters + p,
+                             status, w);
             else if (p == 4)
-                launch_early(k_onesweep_halves<uint32_t, kSrcHigh64, kItems>, tiles, kSortBlock, smem32, stream,
-                    nullptr, vin, keys_in, half[0], vout, n, n_ptr, 0, off, lb, tile_counters + p, status, w);
+                launch_early(early, k_onesweep_halves<uint32_t, kSrcHigh64, kItems>, tiles, kSortBlock, smem32, stream,
+                             nullptr, vin, keys_in, half[0], vout, n, n_ptr, 0, off, lb, tile_counters + p, status, w);
             else if (p == P - 1 && whole_keys)
-                launch_early(k_onesweep_halves<uint64_t, kSrcFull64, kItems>, tiles, kSortBlock, smem64, stream,
-                    nullptr, vin, keys_in, keys_out, vout, n, n_ptr, 8 * p, off, lb, tile_counters + p, status, w);
+                launch_early(early, k_onesweep_halves<uint64_t, kSrcFull64, kItems>, tiles, kSortBlock, smem64, stream,
+                             nullptr, vin, keys_in, keys_out, vout, n, n_ptr, 8 * p, off, lb, tile_counters + p,
+                             status, w);
             else
-                launch_early(k_onesweep_halves<uint32_t, kSrcKeys, kItems>, tiles, kSortBlock, smem32, stream,
-                    half[(p + 1) & 1], vin, nullptr, half[p & 1], vout, n, n_ptr, 8 * (p & 3), off, lb,
-                    tile_counters + p, status, w);
+                launch_early(early, k_onesweep_halves<uint32_t, kSrcKeys, kItems>, tiles, kSortBlock, smem32, stream,
+                             half[(p + 1) & 1], vin, nullptr, half[p & 1], vout, n, n_ptr, 8 * (p & 3), off, lb,
+                             tile_counters + p, status, w);
         };
         if (prof) {
             ProfScope ps(K_ONESWEEP, stream);
@@ -429,8 +439,8 @@ inline int onesweep_launch_t(const K* kin, const uint32_t* vin, K* kout, uint32_
     const size_t smem = onesweep_smem<K>(kItems);
     CPT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, kFirst, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-    launch_early(k_onesweep<K, kFirst, kItems>, sort_tiles(cap), kSortBlock, smem, stream, kin, vin, kout, vout, n, n_ptr,
-                 shift, offsets, lookback, tile_counter, status, wait);
+    launch_early(start_early(cap), k_onesweep<K, kFirst, kItems>, sort_tiles(cap), kSortBlock, smem, stream, kin, vin,
+                 kout, vout, n, n_ptr, shift, offsets, lookback, tile_counter, status, wait);
     CPT_LAUNCH_CHECK();
     return CPT_OK;
 }

@@ -1035,7 +1035,7 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
     k_split_emit<K><<<eblocks, kSplitBlock, 0, stream>>>(bvh->tris, n, s.counts, owner, s.n_pieces, bvh->node_boxes,
                                                          s.pieces, s.keys[0], s.hist, s.zero, s.zero_words);
     CPT_LAUNCH_CHECK();
-    launch_early(k_scan_offsets, P, kRadix, 0, stream, s.hist, s.offsets);
+    launch_early(start_early(cap), k_scan_offsets, P, kRadix, 0, stream, s.hist, s.offsets);
     CPT_LAUNCH_CHECK();
     const uint32_t tiles = sort_tiles(cap);
     uint32_t* lookback = s.zero + 32;
@@ -1072,9 +1072,11 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
     const TreeList list{s.vals[P & 1], reinterpret_cast<uint32_t*>(keys == s.keys[0] ? s.keys[1] : s.keys[0]),
                         s.zero + kTreeListWord};
     const uint32_t blocks = (cap + kTreeBlock - 1) / kTreeBlock;
-    launch_early(k_split_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list, s.n_pieces, cap - 1);
+    launch_early(start_early(cap), k_split_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list, s.n_pieces,
+                 cap - 1);
     CPT_LAUNCH_CHECK();
-    launch_early(k_split_tree_top<K>, tree_top_blocks(blocks, sm_count()), 128, 0, stream, T, leaf, list, s.n_pieces);
+    launch_early(start_early(cap), k_split_tree_top<K>, tree_top_blocks(blocks, sm_count()), 128, 0, stream, T, leaf, list,
+                 s.n_pieces);
     CPT_LAUNCH_CHECK();
     if (treelet) {
         for (int round = 0; round < kTreeletRounds; ++round) {
