@@ -368,6 +368,8 @@ int build_impl(const cpt_triangle* tris_in, uint32_t n, const float* host_box, c
     const uint32_t blocks = (n + kTreeBlock - 1) / kTreeBlock;
     {
         CPT_PROF(K_TOPOLOGY, stream);
+        CPT_CUDA_TRY(cudaFuncSetAttribute(k_tree_blocks<K>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          kTreeCarveout));
         launch_early(start_early(n), k_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list);
     }
     CPT_LAUNCH_CHECK();

@@ -127,6 +127,11 @@ __device__ __forceinline__ int arrive_acq_rel(int* counter)
 constexpr int kTreeBlock = 256;
 constexpr int kTreeLevels = 9;  // tables of 1, 2, ... 256 in a row
 constexpr int kNoEnd = -1;      // ends[g]: no child of split g has arrived
+// Percent of an SM's shared memory that the tree kernels ask for: four blocks instead of five, so
+// that the split is the renderer's and an SM that traces on another stream need not fall idle to
+// change it (C2 frames with the next scene's builds beside them: 135.9 ms a step with five blocks,
+// 122.2 with 71 %, 122.5 with 57 %; the build alone 1.30, 1.35 and 1.35 ms in the same program).
+constexpr int kTreeCarveout = 71;
 constexpr int kTreeListWord = 16;  // the list's count among the 32 zeroed tile counters (a sort uses 9 at most)
 
 // Blocks of 128 threads for tree_climb over the subtrees of `blocks` blocks (a grid-stride

@@ -1072,6 +1072,8 @@ int split_impl(cpt_bvh* bvh, uint32_t cap, bool treelet, void* nodes, void* scra
     const TreeList list{s.vals[P & 1], reinterpret_cast<uint32_t*>(keys == s.keys[0] ? s.keys[1] : s.keys[0]),
                         s.zero + kTreeListWord};
     const uint32_t blocks = (cap + kTreeBlock - 1) / kTreeBlock;
+    CPT_CUDA_TRY(cudaFuncSetAttribute(k_split_tree_blocks<K>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      kTreeCarveout));
     launch_early(start_early(cap), k_split_tree_blocks<K>, blocks, kTreeBlock, 0, stream, T, leaf, list, s.n_pieces,
                  cap - 1);
     CPT_LAUNCH_CHECK();
