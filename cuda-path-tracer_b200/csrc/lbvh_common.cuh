@@ -115,7 +115,9 @@ __device__ __forceinline__ int arrive_acq_rel(int* counter)
 // exchange (which also publishes and acquires the boxes) and makes the node.
 //
 // A node's box is the union of its leaves in order, each bound the last of equal ones (glm's
-// min and max select their second argument), so the grouping does not show in the bytes.
+// min and max select their second argument), so the grouping does not show in the bytes — unless
+// a bound is NaN: then min(a, min(NaN, c)) is not min(min(a, NaN), c), and a block that holds one
+// unites its boxes child by child instead (Leaf::kAnyGrouping: a union that ignores NaN).
 //
 // 5.24 M triangles (1.22 GB of DRAM traffic): 724 us as a launch of key searches per node and
 // a walk per leaf through the records in memory (a third of the lanes left at every level, 25 %
@@ -205,6 +207,7 @@ __device__ __forceinline__ void tree_block(TreeSmem& sm, const TreeArrays<K>& T,
         sm.least[0][h] = (uint8_t)d;
     }
     float bx[6];
+    bool unordered = false;
     if (t < nb) {
         float slot[10];
         leaf.load(base + (uint32_t)t, slot, bx);
@@ -212,9 +215,12 @@ __device__ __forceinline__ void tree_block(TreeSmem& sm, const TreeArrays<K>& T,
         for (int k = 0; k < 10; ++k) sm.slot[t][k] = slot[k];
         sm.row[0][0][t] = make_float4(bx[0], bx[1], bx[2], 0.f);
         sm.row[0][1][t] = make_float4(bx[3], bx[4], bx[5], 0.f);
+        if (!Leaf::kAnyGrouping)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) unordered = unordered || bx[c] != bx[c];
     }
     sm.made[t] = 0;
-    __syncthreads();
+    unordered = __syncthreads_or(unordered);
 #pragma unroll
     for (int k = 1; k < kTreeLevels; ++k) {
         const int o = 1 << (k - 1);
@@ -240,11 +246,31 @@ __device__ __forceinline__ void tree_block(TreeSmem& sm, const TreeArrays<K>& T,
     }
     sm.whole[t] = node;
     if (t < nb && !node && (int)base + t + 1 < n) T.ends[base + (uint32_t)t] = kNoEnd;
-    // boxes: a range of len leaves is the union of its first and its last 2^k, 2^k <= len < 2^(k + 1)
+    const int at = node ? (sm.least[0][hi + 1] > sm.least[0][lo] ? hi : lo) : 0;
     float nbx[6];
+    if (unordered) {  // child by child, a node when both its children are there (node t's: t and t + 1)
+        bool todo = node;
+        while (__syncthreads_or(todo)) {
+            const bool ready = todo && (lo == t || sm.made[t]) && (hi == t + 1 || sm.made[t + 1]);
+            __syncthreads();
+            if (ready) {
+                const float4 a = sm.row[0][0][t], b = sm.row[0][1][t], c = sm.row[0][0][t + 1], d = sm.row[0][1][t + 1];
+                const float lf[6] = {a.x, a.y, a.z, b.x, b.y, b.z}, rf[6] = {c.x, c.y, c.z, d.x, d.y, d.z};
+#pragma unroll
+                for (int c6 = 0; c6 < 6; ++c6) {
+                    const float l6 = lo == t ? lf[c6] : sm.box[t][c6], r6 = hi == t + 1 ? rf[c6] : sm.box[t + 1][c6];
+                    nbx[c6] = c6 < 3 ? Leaf::lo(l6, r6) : Leaf::hi(l6, r6);
+                    sm.box[at][c6] = nbx[c6];
+                }
+                sm.made[at] = 1;
+                todo = false;
+            }
+        }
+    }
+    // boxes: a range of len leaves is the union of its first and its last 2^k, 2^k <= len < 2^(k + 1)
     const int mine = node ? 31 - __clz(hi - lo + 1) : -1;
 #pragma unroll 1
-    for (int k = 0; k < kTreeLevels; ++k) {
+    for (int k = 0; k < kTreeLevels && !unordered; ++k) {
         const float4(*row)[kTreeBlock] = sm.row[k & 1];
         float4(*next)[kTreeBlock] = sm.row[(k + 1) & 1];
         const int w = 1 << k;
@@ -263,9 +289,7 @@ __device__ __forceinline__ void tree_block(TreeSmem& sm, const TreeArrays<K>& T,
         if (!__syncthreads_or(mine > k)) break;
     }
     __syncthreads();  // the rows give way to the records
-    int at = 0;
     if (node) {
-        at = sm.least[0][hi + 1] > sm.least[0][lo] ? hi : lo;
         sm.made[at] = 1;
 #pragma unroll
         for (int c = 0; c < 6; ++c) sm.box[at][c] = nbx[c];
@@ -421,6 +445,7 @@ struct TriangleLeaves {
     float* tris_out;
     uint32_t* status;
 
+    static constexpr bool kAnyGrouping = false;
     static __device__ __forceinline__ float lo(float a, float b) { return gmin(a, b); }
     static __device__ __forceinline__ float hi(float a, float b) { return gmax(a, b); }
     static __device__ __forceinline__ void make(uint32_t i, const float2 v2[5], float slot[10], float box[6])

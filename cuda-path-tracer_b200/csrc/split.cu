@@ -421,6 +421,7 @@ struct PieceLeaves {
     uint32_t n, n_tris;
     uint32_t* status;
 
+    static constexpr bool kAnyGrouping = true;
     static __device__ __forceinline__ float lo(float a, float b) { return fminf(a, b); }
     static __device__ __forceinline__ float hi(float a, float b) { return fmaxf(a, b); }
     __device__ __forceinline__ void get(uint32_t i, float slot[10], float4& a, float4& b) const
