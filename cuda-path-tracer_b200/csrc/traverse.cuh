@@ -451,10 +451,29 @@ __device__ __forceinline__ uint2 wide_pop(const uint2* smem_col, const uint2* sp
     return sp < kWideSmemStack ? smem_col[sp * kBlock] : spill[sp - kWideSmemStack];
 }
 
+// The distance at which the ray enters the box of one slot of a wide node, as wide_child_hits
+// computes it (the same roundings).
+__device__ __forceinline__ float wide_slot_entry(const WideState& s, const float4* nd, uint32_t slot)
+{
+    const float4 n0 = __ldg(nd);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(nd) + (slot >> 1);
+    const uint32_t h01 = __ldg(reinterpret_cast<const uint32_t*>(nd) + 7), h2 = __float_as_uint(n0.w);
+    const uint32_t shift = 16u * (slot & 1u);
+    auto plane = [&](uint32_t word, uint32_t negative, float scale, float p, float o, float dinv) {
+        const float a = __fmul_rn(scale, dinv);
+        const float b = fmaf(-1024.0f, a, __fmul_rn(__fsub_rn(p, o), dinv));
+        return fmaf(1024.0f + (float)((word >> (shift + (negative ? 8u : 0u))) & 255u), a, b);
+    };
+    return fmaxf(fmax3(plane(__ldg(w + 8), s.oct & 1u, __uint_as_float(h01 << 16), n0.x, s.o.x, s.dinv.x),
+                       plane(__ldg(w + 12), s.oct & 2u, __uint_as_float(h01 & 0xFFFF0000u), n0.y, s.o.y, s.dinv.y),
+                       plane(__ldg(w + 16), s.oct & 4u, __uint_as_float(h2 << 16), n0.z, s.o.z, s.dinv.z)),
+                 0.0f);
+}
+
 // The children of a wide node (five float4 n0..n4) whose boxes the ray's interval
-// [0, best] meets: bit i for slot i.
+// [0, tlim] meets: bit i for slot i.
 __device__ __forceinline__ uint32_t wide_child_hits(const WideState& s, float4 n0, float4 n1, float4 n2, float4 n3,
-                                                    float4 n4)
+                                                    float4 n4, float tlim)
 {
     // per-axis scales 2^e: the float bits e << 23 are stored as half-words (x, y in n1.w,
     // z in the low half of n0.w), moved to the high half by one byte permute each
@@ -480,7 +499,6 @@ __device__ __forceinline__ uint32_t wide_child_hits(const WideState& s, float4 n
     const uint32_t px0 = (oct & 1u) ? 0x4041u : 0x4140u, py0 = (oct & 2u) ? 0x4041u : 0x4140u,
                    pz0 = (oct & 4u) ? 0x4041u : 0x4140u;
     const uint32_t sel[2][3] = {{px0, py0, pz0}, {px0 + 0x0202u, py0 + 0x0202u, pz0 + 0x0202u}};
-    const float tlim = s.t;
     uint32_t hm = 0;
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {  // two children at a time
@@ -505,16 +523,24 @@ __device__ __forceinline__ uint32_t wide_child_hits(const WideState& s, float4 n
     return hm;
 }
 
+struct WideNoTail {
+    __device__ __forceinline__ void other(float, float) const {}
+    __device__ __forceinline__ void queued(int, uint32_t) const {}
+    __device__ __forceinline__ void move_up() const {}
+    __device__ __forceinline__ float behind(float t) const { return t; }
+};
+
 // One step; returns true when the ray is finished.
 // perm: xor_permute8 as a table in shared memory, byte oct * 256 + x (wide_perm_table).
 // bot: the lowest stack entry still the lane's own (above 0 once others have been given
 // away from the bottom; see wide_tail).
-// hit(t, u, v, triangle): a nearer hit than any before (kAny: the hit). tie(triangle): a
-// triangle at exactly the nearest hit's distance.
-template <bool kAny, int kBlock, bool kStats, typename OnHit, typename OnTie>
+// hit(t, u, v, triangle, slot): a nearer hit than any before (kAny: the hit), in leaf slot `slot`
+// of the first triangle group's node.
+// tail: what a step among lanes that share rays adds (WideShareTail).
+template <bool kAny, int kBlock, bool kStats, typename OnHit, typename Tail = WideNoTail>
 __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* spill, bool& overflow,
                                           uint32_t& n_nodes, uint32_t& n_tris, const uint8_t* perm, OnHit hit,
-                                          OnTie tie, bool test_tri = true, int bot = 0)
+                                          bool test_tri = true, int bot = 0, const Tail& tail = Tail())
 {
     if (test_tri && (s.tbits & kWideRecBits)) {
         // the lowest record bit, 8j + slot (the leaf mask lies above): record j * L + rank
@@ -532,10 +558,10 @@ __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* 
         if (kStats) { ++n_tris; ++s.tests; }
         if (t < s.t) {
             s.t = kAny ? kWideFound : t;
-            hit(t, u, v, a.w);
+            hit(t, u, v, a.w, (uint32_t)__popc(below) & 7u);
             if (kAny) return true;
-        } else if (t == s.t) {
-            tie(a.w);
+        } else {
+            tail.other(t, a.w);
         }
         if (!(s.tbits & kWideRecBits) && (s.tbits2 & kWideRecBits)) {  // the queued groups move up
             s.tbase = s.tbase2;
@@ -543,6 +569,7 @@ __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* 
             s.tbase2 = s.tbase3;
             s.tbits2 = s.tbits3;
             s.tbits3 = 0;
+            tail.move_up();
         }
         if (s.tbits3 & kWideRecBits) return false;  // every group slot pending: no node visit this step
     }
@@ -562,7 +589,7 @@ __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* 
     const float4* nd = s.nodes + 5 * (size_t)child;
     const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3), n4 = __ldg(nd + 4);
     const uint32_t imask = __float_as_uint(n0.w) >> 24, lw = __float_as_uint(n1.z);
-    const uint32_t hm = wide_child_hits(s, n0, n1, n2, n3, n4);
+    const uint32_t hm = wide_child_hits(s, n0, n1, n2, n3, n4, tail.behind(s.t));
     s.cbase = __float_as_uint(n1.x);
     s.gbits = (uint32_t)perm[(s.oct << 8) | (hm & imask)] | (imask << 8);
     // the hit slots' records: the hit mask copied into bytes 0-2, masked by the slots
@@ -572,14 +599,17 @@ __device__ __forceinline__ bool wide_step(WideState& s, uint2* smem_col, uint2* 
         if (s.tbits2 & kWideRecBits) {
             s.tbase3 = __float_as_uint(n1.y);
             s.tbits3 = recs;
+            tail.queued(2, child);
             return false;
         }
         s.tbase2 = __float_as_uint(n1.y);
         s.tbits2 = recs;
+        tail.queued(1, child);
         return false;
     }
     s.tbase = __float_as_uint(n1.y);
     s.tbits = recs;
+    tail.queued(0, child);
     return false;
 }
 
@@ -696,21 +726,61 @@ __device__ __forceinline__ uint32_t wide_ray_lanes(uint32_t n)
 // the state live across the loop's end, C2 ran 5 to 8 % slower. For the same reason a hit is
 // written when it is found instead of carried (u, v, triangle) to the ray's end.
 //
-// The hit is the one that a lane finds alone: a child box is wide enough that no order of
-// visits loses a hit (the binary trees' boxes are not, and their traversal keeps the
-// reference's order), and a ray that meets two triangles at exactly its nearest distance,
-// of which a lane alone reports the one it visits first, is traced anew by its own lane
-// alone (two or three rays of a million; from the start, since a split triangle may be met
-// first through the box of a piece that does not hold the hit). Every iteration each working
-// lane consumes a node, a stack entry or a triangle, as in the main loop; a helper goes on
-// counting its donor's node visits and the iterations are limited, so that a corrupt tree
-// ends in an overflow report.
+// The hit is the one that a lane finds alone, one visit after the other. Which boxes are passed
+// over depends on what has been found by then, and the distance that tri_test computes for a
+// thin triangle can lie before the box that holds it, by more than the box's margin (hairballs:
+// 0.05 % of hits from 3.6 units away, 0.3 % from 20, 1.3 % from 100). So while lanes share a ray,
+//  * a box is passed over only behind kWideBehind times the nearest hit: no lane misses a
+//    triangle that one alone would have met before it found that hit;
+//  * the nearest hit comes with its box's entry, and with the next nearest triangle met. A lane
+//    alone may have passed over that box only if it knew of a hit before the box's entry: then,
+//    and if two triangles lie at exactly the nearest distance (of which a lane alone reports the
+//    one it visits first), the ray is traced anew by its own lane alone (a few rays of a million;
+//    from the start, since a split triangle may be met first through the box of a piece that does
+//    not hold the hit).
+// What is left to chance is a triangle computed nearer than its box by 1/64 of its distance, or
+// than a box above its own by less than that box's quantum; and, with lanes sharing or not, when
+// in a warp's batch of triangle tests its turn comes (400,000 hairs from 400 units: 1 of 20,000
+// rays in every run without these rules, 0 of 13 M with them; the counting traversal, which
+// shares nothing, 3 of 13 M). They cost the frames above 0.5 to 3 %.
+// Every iteration each working lane consumes a node, a stack entry or a triangle, as in the main
+// loop; a helper goes on counting its donor's node visits and the iterations are limited, so that
+// a corrupt tree ends in an overflow report.
 constexpr int kWideTailLanes = 12;
-struct WideTail {  // per warp, in shared memory
-    int t[32];          // float bits of the ray's nearest distance (as int: -0 and kWideFound sort lowest)
+struct WideTail {  // per warp, in shared memory; t to other by the ray's lane
+    float t[32];        // the ray's nearest distance
     uint32_t tri[32];   // the triangle there
-    uint32_t info[32];  // byte 0: helpers at work; byte 1 (of word r): the r-th lane with a stack entry to give;
-                        // bit 31: another triangle lies at exactly the nearest distance
+    float entry[32];    // the entry of its box (0: found by the ray's own lane)
+    float other[32];    // the nearest distance of another triangle
+    uint32_t info[32];  // byte 0: helpers at work; byte 1 (of word r): the r-th lane with a stack entry to give
+};
+constexpr float kWideBehind = 1.0f + 1.0f / 64.0f;  // (1/256 costs as much; 0: 3 of 640,000 rays differ from 400 units)
+constexpr int kWideSpill = CPT_TRAVERSAL_STACK - kWideSmemStack;
+// A lane's words that are rarely touched: in local memory, behind its stack, so that they hold no
+// register while a node is visited.
+struct WideLaneTail {
+    uint32_t node[3];           // the nodes of its triangle groups (invalid: from before the lanes shared)
+    float t, u, v, tri, entry;  // the triangle met in this step, the entry of its box
+};
+static_assert(sizeof(WideLaneTail) % sizeof(uint2) == 0, "whole stack entries");
+
+// A step of wide_tail: the other triangles met (t, triangle), the nodes of the triangle groups
+// queued at position k, and the distance from which boxes are passed over.
+struct WideShareTail {
+    WideLaneTail& l;
+    bool& seen;
+    bool exact;
+    __device__ __forceinline__ void other(float t, float tri) const
+    {
+        if (t < FLT_MAX) { seen = true; l.t = t; l.tri = tri; }
+    }
+    __device__ __forceinline__ void queued(int k, uint32_t n) const { l.node[k] = n; }
+    __device__ __forceinline__ void move_up() const
+    {
+        l.node[0] = l.node[1];
+        l.node[1] = l.node[2];
+    }
+    __device__ __forceinline__ float behind(float t) const { return exact ? t : t * kWideBehind; }
 };
 
 template <bool kAny, int kBlock, typename Sink>
@@ -725,23 +795,28 @@ __device__ __noinline__ bool wide_tail(WideState s, uint32_t ray, uint2* smem_co
     bool overflow = false;
     int bot = 0;
     uint32_t nn = 0, nt = 0;
-    constexpr uint32_t kTie = 0x80000000u;
+    WideLaneTail& mine = *reinterpret_cast<WideLaneTail*>(spill + kWideSpill);
     bool alone = false;  // a ray traced anew: its lane gives nothing away
     // more steps than the longest valid traversal takes: its nodes and their records
-    uint32_t limit = __reduce_max_sync(0xFFFFFFFFu, work ? s.max_visits : 0u);
-    limit = limit < (1u << 26) ? 32u * limit + 1024u : 0x80000000u;
+    uint32_t left = __reduce_max_sync(0xFFFFFFFFu, work ? s.max_visits : 0u);
+    left = left < (1u << 26) ? 32u * left + 1024u : 0x80000000u;
     bool share = false;  // until kWideTailLanes lanes are left, each traces its own ray as in the main loop
 #pragma unroll 1
-    for (uint32_t iter = 0;; ++iter) {
+    for (;; left -= left ? 1u : 0u) {
         const unsigned wm = __ballot_sync(0xFFFFFFFFu, work);
         if (wm == 0u) break;
         bool test_tri = true;
         if (!share) {
             if (__popc(wm) <= kWideTailLanes) {
                 share = true;
-                w.t[lane] = __float_as_int(s.t);
+                w.t[lane] = s.t;
                 w.info[lane] = 0;
-                if (!kAny && work && s.t < FLT_MAX) w.tri[lane] = sink.found(ray);
+                if (!kAny) {
+                    w.tri[lane] = work && s.t < FLT_MAX ? sink.found(ray) : CPT_INVALID_INDEX;
+                    w.entry[lane] = 0.0f;
+                    w.other[lane] = FLT_MAX;
+                    mine.node[0] = mine.node[1] = mine.node[2] = CPT_INVALID_INDEX;
+                }
                 __syncwarp();
             } else {
                 test_tri = wide_test_now(s, work);
@@ -790,26 +865,29 @@ __device__ __noinline__ bool wide_tail(WideState s, uint32_t ray, uint2* smem_co
             }
             __syncwarp();
         }
-        bool fin = false, found = false;
-        float hu = 0.f, hv = 0.f, htri = 0.f, ht = 0.f;
+        bool fin = false, found = false, seen = false;
         if (work) {
-            fin = wide_step<kAny, kBlock, false>(
-                s, smem_col, spill, overflow, nn, nt, perm,
-                [&](float t, float u, float v, float tri) {
-                    if (share) {
-                        found = true;
-                        ht = t; hu = u; hv = v; htri = tri;
-                    } else {
-                        sink.hit(ray, t, u, v, tri);
-                    }
-                },
-                [&](float tri) {
-                    if (!kAny && share && s.t < FLT_MAX && w.tri[owner] != __float_as_uint(tri))
-                        atomicOr(&w.info[owner], kTie);
-                },
-                test_tri, bot);
-            if (found) atomicMin(&w.t[owner], __float_as_int(s.t));
-            if (iter >= limit) { overflow = true; fin = true; }
+            auto hit = [&](float t, float u, float v, float tri, uint32_t slot) {
+                if (kAny || !share) {
+                    sink.hit(target, t, u, v, tri);
+                    found = true;
+                } else {
+                    seen = true;
+                    mine.t = t;
+                    mine.u = u;
+                    mine.v = v;
+                    mine.tri = tri;
+                    const uint32_t node = mine.node[0];
+                    mine.entry = node != CPT_INVALID_INDEX ? wide_slot_entry(s, s.nodes + 5 * (size_t)node, slot) : 0.0f;
+                }
+            };
+            if constexpr (kAny)
+                fin = wide_step<kAny, kBlock, false>(s, smem_col, spill, overflow, nn, nt, perm, hit, test_tri, bot);
+            else
+                fin = wide_step<kAny, kBlock, false>(
+                    s, smem_col, spill, overflow, nn, nt, perm, hit, test_tri, bot,
+                    WideShareTail{mine, seen, !share || alone});
+            if (left == 0u) { overflow = true; fin = true; }
         }
         if (!share) {
             if (fin) {
@@ -819,31 +897,35 @@ __device__ __noinline__ bool wide_tail(WideState s, uint32_t ray, uint2* smem_co
             }
             continue;
         }
-        __syncwarp();
-        if (work || ray != CPT_INVALID_INDEX) {
-            const float near = __int_as_float(*reinterpret_cast<volatile int*>(&w.t[owner]));
-            found = found && near == s.t;
-            s.t = near;
-            if (kAny && near == kWideFound) fin = work;
-        }
-        // nearer hits are reported one lane after the other; of several at one distance the
-        // first is, and the tie noted
-        for (unsigned hm = __ballot_sync(0xFFFFFFFFu, found), seen = 0; hm; hm &= hm - 1u) {
-            const int l = __ffs(hm) - 1;
-            const uint32_t ow = __shfl_sync(0xFFFFFFFFu, owner, l);
-            if ((int)lane == l) {
-                if ((seen >> ow) & 1u) {
-                    if (!kAny && w.tri[ow] != __float_as_uint(htri)) atomicOr(&w.info[ow], kTie);
-                } else {
-                    if (!kAny) {
-                        w.tri[ow] = __float_as_uint(htri);
-                        atomicAnd(&w.info[ow], ~kTie);
-                    }
-                    sink.hit(target, ht, hu, hv, htri);
-                }
-            }
-            seen |= 1u << ow;
+        if (kAny) {
+            if (found) w.t[owner] = kWideFound;
             __syncwarp();
+            if ((work || ray != CPT_INVALID_INDEX) && *reinterpret_cast<volatile float*>(&w.t[owner]) == kWideFound) {
+                s.t = kWideFound;
+                fin = work;
+            }
+        } else {
+            // the triangles met are reported one lane after the other
+            unsigned hm = __ballot_sync(0xFFFFFFFFu, seen);
+            if (hm) {
+                do {
+                    if ((int)lane == __ffs(hm) - 1) {
+                        const float t = w.t[owner];
+                        if (mine.t < t) {
+                            w.other[owner] = t;
+                            w.t[owner] = mine.t;
+                            w.tri[owner] = __float_as_uint(mine.tri);
+                            w.entry[owner] = mine.entry;
+                            sink.hit(target, mine.t, mine.u, mine.v, mine.tri);
+                        } else if (w.tri[owner] != __float_as_uint(mine.tri)) {
+                            w.other[owner] = fminf(w.other[owner], mine.t);
+                        }
+                    }
+                    __syncwarp();
+                    hm &= hm - 1u;
+                } while (hm);
+                s.t = w.t[owner];
+            }
         }
         if (fin) {
             work = false;
@@ -851,12 +933,13 @@ __device__ __noinline__ bool wide_tail(WideState s, uint32_t ray, uint2* smem_co
         }
         __syncwarp();
         if (ray != CPT_INVALID_INDEX && !work && (w.info[lane] & 0xFFu) == 0u) {
-            if (!kAny && (w.info[lane] & kTie) && !alone) {
+            const float other = kAny ? FLT_MAX : w.other[lane];
+            if (!kAny && !alone && s.t < FLT_MAX && (other == s.t || w.entry[lane] > __fmul_rn(other, kWideGrow))) {
                 const float4* nodes = s.nodes;
                 wide_init(s, nodes, s.tris, s.max_visits, s.o, s.d);
                 bot = 0;
                 alone = work = true;
-                w.t[lane] = __float_as_int(s.t);
+                w.t[lane] = s.t;
             } else {
                 sink.done(ray, s);
                 ray = CPT_INVALID_INDEX;
@@ -899,7 +982,7 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
     const uint32_t lt_mask = (1u << lane) - 1u;
     __shared__ uint8_t s_perm[2048];
     wide_perm_table(s_perm);
-    uint2 spill[CPT_TRAVERSAL_STACK - kWideSmemStack];
+    uint2 spill[kWideSpill + (kTail ? sizeof(WideLaneTail) / sizeof(uint2) : 0)];
     WideState s;
     uint32_t ray = CPT_INVALID_INDEX;
     bool drained = false;
@@ -944,7 +1027,7 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
             if (ray != CPT_INVALID_INDEX &&
                 wide_step<kAny, kBlock, kStats>(
                     s, smem_col, spill, overflow, n_nodes, n_tris, s_perm,
-                    [&](float t, float u, float v, float tri) { sink.hit(ray, t, u, v, tri); }, [](float) {}, test_tri)) {
+                    [&](float t, float u, float v, float tri, uint32_t) { sink.hit(ray, t, u, v, tri); }, test_tri)) {
                 sink.done(ray, s);
                 ray = CPT_INVALID_INDEX;
             }
