@@ -282,13 +282,14 @@ constexpr int kViewsRefillLanes = 28;
 #endif
 // kWide: every view's wide tree (cpt_lbvh_wide) instead of its binary nodes.
 static_assert(kWideSmemStack * 2 <= kSmemStack, "wide and binary stacks share the shared-memory buffer");
-template <bool kStats, bool kOneView, bool kWide>
+// kTail: its launches share their last rays among lanes (wide_share).
+template <bool kStats, bool kOneView, bool kWide, bool kTail = false>
 __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(Views vs, const float4* __restrict__ queue,
                                                          const uint32_t* __restrict__ count, float4* __restrict__ hits,
                                                          uint32_t* __restrict__ pool,
                                                          unsigned long long* __restrict__ ray_counts,
                                                          uint32_t* __restrict__ status, const uint32_t* __restrict__ order,
-                                                         uint32_t refill)
+                                                         uint32_t refill, uint32_t spread)
 {
     __shared__ __align__(16) uint32_t s_stack[(kWide ? 2 * kWideSmemStack : kSmemStack) * kExtendBlock];
     const uint32_t n = *count;
@@ -308,9 +309,9 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(
             tr = vs.v[vi].wide_tris;
             return vs.v[vi].wide_nodes;
         };
-        persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false, !kStats>(
+        persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false, kTail>(
             wide_of, queue, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, order,
-            WideHits{hits}, refill ? refill : kOneView ? (uint32_t)kWideRefillLanes : (uint32_t)kViewsRefillLanes);
+            WideHits{hits}, spread, refill ? refill : kOneView ? (uint32_t)kWideRefillLanes : (uint32_t)kViewsRefillLanes);
         if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
         if (kStats && ray_counts) {
             warp_count_u64(ray_counts + 3, nn);
@@ -669,12 +670,12 @@ struct Unoccluded {
 // Shadow rays of next-event estimation: any-hit up to each ray's far limit; an
 // unoccluded ray adds its emission to its path's radiance (one shadow ray per
 // path and vertex, so no two threads add to the same path).
-template <bool kOneView, bool kWide>
+template <bool kOneView, bool kWide, bool kTail = false>
 __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_occlude(Views vs, const float4* __restrict__ rays,
                                                           const float4* __restrict__ emission,
                                                           const uint32_t* __restrict__ count,
                                                           uint32_t* __restrict__ pool, float4* __restrict__ state,
-                                                          uint32_t* __restrict__ status)
+                                                          uint32_t* __restrict__ status, uint32_t spread)
 {
     __shared__ __align__(16) uint32_t s_stack[(kWide ? 2 * kWideSmemStack : kSmemStack) * kExtendBlock];
     const uint32_t n = *count;
@@ -687,9 +688,9 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_occlude
             tr = vs.v[v].wide_tris;
             return vs.v[v].wide_nodes;
         };
-        persistent_trace_wide<true, kExtendBlock, false, kExtendSteps, true, true>(
+        persistent_trace_wide<true, kExtendBlock, false, kExtendSteps, true, kTail>(
             wide_of, rays, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, nullptr,
-            Unoccluded{emission, state});
+            Unoccluded{emission, state}, spread);
         if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
         return;
     }
@@ -1075,6 +1076,8 @@ int render_views(const Views& vs, bool any_lights, const cpt_bbox* sort_root, co
     for (uint32_t i = 1; i < vs.n; ++i) one_bvh &= vs.v[i].nodes == vs.v[0].nodes;
     for (uint32_t i = 0; i < vs.n; ++i) wide &= vs.v[i].wide_nodes != nullptr;  // else every view's binary tree
     const int sms = sm_count();
+    uint32_t leaves = 0;
+    for (uint32_t i = 0; i < vs.n; ++i) leaves = std::max(leaves, vs.v[i].wide_cap + 1u);
     static int ext_occ = 0;
     if (!ext_occ) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ext_occ, k_extend<false, false, false>, kExtendBlock, 0) != cudaSuccess ||
@@ -1112,7 +1115,9 @@ int render_views(const Views& vs, bool any_lights, const cpt_bbox* sort_root, co
                          st>>>(wl, vs, L.queue[0], L.counts, rs.state);
         }
         CPT_LAUNCH_CHECK();
-        const uint32_t block_rays = wide ? (uint32_t)(kWideMinLanes * kExtendBlock / 32) : (uint32_t)kExtendBlock;
+        // (a launch has up to `paths` rays, and blocks for as many as may be spread)
+        const WideShare share = wide ? wide_share(leaves, sms) : WideShare{false, 0u};
+        const uint32_t block_rays = wide_block_rays(share, 1u, kExtendBlock);
         const int ext_blocks = std::min<int>((int)((paths + block_rays - 1) / block_rays), sms * per_sm);
         const int shade_blocks = std::min<int>((int)((paths + kShadeBlock - 1) / kShadeBlock), sms * 16);
         for (uint32_t b = 0; b <= params->bounces; ++b) {
@@ -1128,12 +1133,14 @@ int render_views(const Views& vs, bool any_lights, const cpt_bbox* sort_root, co
             {
                 CPT_PROF(K_EXTEND, st);
                 uint32_t* pool = L.counts + kMaxDepth + 2 + b;
-#define CPT_EXTEND(S, O, W) \
-    k_extend<S, O, W><<<ext_blocks, kExtendBlock, 0, st>>>(vs, qin, L.counts + b, L.hits, pool, ray_counts, status, \
-                                                           order, refill)
+#define CPT_EXTEND(S, O, ...) \
+    k_extend<S, O, __VA_ARGS__><<<ext_blocks, kExtendBlock, 0, st>>>(vs, qin, L.counts + b, L.hits, pool, ray_counts, status, \
+                                                           order, refill, share.spread)
                 if (wide) {
                     if (params->trace_stats) {
                         if (one_bvh) CPT_EXTEND(true, true, true); else CPT_EXTEND(true, false, true);
+                    } else if (share.tail) {
+                        if (one_bvh) CPT_EXTEND(false, true, true, true); else CPT_EXTEND(false, false, true, true);
                     } else {
                         if (one_bvh) CPT_EXTEND(false, true, true); else CPT_EXTEND(false, false, true);
                     }
@@ -1177,10 +1184,12 @@ int render_views(const Views& vs, bool any_lights, const cpt_bbox* sort_root, co
                 CPT_PROF(K_OCCLUDE, st);
                 uint32_t* spool = L.counts + kShadowPoolWord + b;
                 const uint32_t* scount = L.counts + kShadowCountWord + b;
-#define CPT_OCCLUDE(O, W)                                                                                   \
-    k_occlude<O, W><<<ext_blocks, kExtendBlock, 0, st>>>(vs, L.shadow_rays, L.shadow_emission, scount, spool, \
-                                                         rs.state, status)
-                if (wide) {
+#define CPT_OCCLUDE(O, ...)                                                                                 \
+    k_occlude<O, __VA_ARGS__><<<ext_blocks, kExtendBlock, 0, st>>>(vs, L.shadow_rays, L.shadow_emission, scount, spool, \
+                                                         rs.state, status, share.spread)
+                if (wide && share.tail) {
+                    if (one_bvh) CPT_OCCLUDE(true, true, true); else CPT_OCCLUDE(false, true, true);
+                } else if (wide) {
                     if (one_bvh) CPT_OCCLUDE(true, true); else CPT_OCCLUDE(false, true);
                 } else {
                     if (one_bvh) CPT_OCCLUDE(true, false); else CPT_OCCLUDE(false, false);

@@ -54,16 +54,17 @@ template <bool kAny, bool kStats> struct TraceSink : WideHits {
 
 // Closest hits: 8 blocks per SM (64 registers), as the renderer's traversal: left to itself the
 // compiler takes 74 to 85 registers, 5 or 6 blocks, and the latency of the node fetches shows
-// (one million incoherent rays: 3.8 ms at 6 blocks, 2.5 at 8). Visibility and counting rays
-// share no tails, and a launch of 150,000 to 300,000 of them lasts 5 to 20 % longer when all fit
-// at once than when lanes refill: 7 blocks (150,000 visibility rays over 1.2 M triangles 5.46 ms
+// (one million incoherent rays: 3.8 ms at 6 blocks, 2.5 at 8). Where nothing is shared
+// (visibility, counts, tiny trees) a launch of 150,000 to 300,000 rays lasts 5 to 20 % longer
+// when all fit at once than when lanes refill: 7 blocks, 6 for tiny trees (150,000 visibility rays over 1.2 M triangles 5.46 ms
 // at 8, 5.01 at 7, 4.79 at 6; 1,000,003 of them 14.0, 13.9 and 14.3).
-template <bool kAny, bool kStats>
-__global__ void __launch_bounds__(kTraceBlock, kAny || kStats ? 7 : 8) k_trace_wide(const float4* __restrict__ nodes,
+template <bool kAny, bool kStats, bool kTail>
+__global__ void __launch_bounds__(kTraceBlock, kTail ? 8 : kAny || kStats ? 7 : 6) k_trace_wide(const float4* __restrict__ nodes,
                                                             const float4* __restrict__ tris, uint32_t node_cap,
                                                             const float4* __restrict__ rays, uint32_t n,
                                                             float4* __restrict__ hits, uint2* __restrict__ stats,
-                                                            uint32_t* __restrict__ pool, uint32_t* __restrict__ status)
+                                                            uint32_t* __restrict__ pool, uint32_t* __restrict__ status,
+                                                            uint32_t spread)
 {
     __shared__ uint2 s_stack[kWideSmemStack * kTraceBlock];
     bool overflow = false;
@@ -73,29 +74,28 @@ __global__ void __launch_bounds__(kTraceBlock, kAny || kStats ? 7 : 8) k_trace_w
         tr = tris;
         return nodes;
     };
-    persistent_trace_wide<kAny, kTraceBlock, kStats, kTraceSteps, false, !kAny && !kStats>(
+    persistent_trace_wide<kAny, kTraceBlock, kStats, kTraceSteps, false, kTail>(
         wide_of, rays, n, pool, s_stack + threadIdx.x, overflow, nn, nt, nullptr,
-        TraceSink<kAny, kStats>(hits, stats));
+        TraceSink<kAny, kStats>(hits, stats), spread);
     if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
 }
 
-template <bool kAny, bool kStats>
+template <bool kAny, bool kStats, bool kTail>
 int launch_trace_wide(const cpt_bvh* bvh, const float4* r4, uint32_t n, float4* h4, uint2* st, uint32_t* pool,
-                      cudaStream_t stream)
+                      WideShare share, cudaStream_t stream)
 {
-    static int per_sm[2][2] = {{0, 0}, {0, 0}};
-    int& occ = per_sm[kAny][kStats];
+    static int occ = 0;
     if (!occ) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trace_wide<kAny, kStats>, kTraceBlock, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trace_wide<kAny, kStats, kTail>, kTraceBlock, 0) !=
                 cudaSuccess ||
             occ < 1)
             occ = 1;
     }
-    const uint32_t block_rays = !kAny && !kStats ? (uint32_t)(kWideMinLanes * kTraceBlock / 32) : (uint32_t)kTraceBlock;
+    const uint32_t block_rays = wide_block_rays(share, n, kTraceBlock);
     const int blocks = (int)std::min<size_t>((n + block_rays - 1) / block_rays, (size_t)sm_count() * occ);
-    k_trace_wide<kAny, kStats><<<blocks, kTraceBlock, 0, stream>>>(
+    k_trace_wide<kAny, kStats, kTail><<<blocks, kTraceBlock, 0, stream>>>(
         static_cast<const float4*>(bvh->wide_nodes), static_cast<const float4*>(bvh->wide_tris), bvh->wide_capacity - 1,
-        r4, n, h4, st, pool, bvh->status);
+        r4, n, h4, st, pool, bvh->status, share.spread);
     CPT_LAUNCH_CHECK();
     return CPT_OK;
 }
@@ -140,10 +140,15 @@ extern "C" int cpt_trace(const cpt_bvh* bvh, const float* rays, uint32_t n, int 
     const uint32_t mv = bvh->split_nodes ? (bvh->split_capacity | kFastSlabBit) : bvh->n;
     CPT_PROF(K_TRACE, stream);
     if (bvh->wide_nodes) {  // the wide tree when one was built
-        if (any_hit) return stats ? launch_trace_wide<true, true>(bvh, r4, n, h4, st, pool, stream)
-                                  : launch_trace_wide<true, false>(bvh, r4, n, h4, st, pool, stream);
-        return stats ? launch_trace_wide<false, true>(bvh, r4, n, h4, st, pool, stream)
-                     : launch_trace_wide<false, false>(bvh, r4, n, h4, st, pool, stream);
+        const WideShare none{false, 0u}, share = any_hit || stats ? none : wide_share(bvh->wide_capacity, sm_count());
+        if (any_hit) return stats ? launch_trace_wide<true, true, false>(bvh, r4, n, h4, st, pool, none, stream)
+                                  : launch_trace_wide<true, false, false>(bvh, r4, n, h4, st, pool, none, stream);
+        if (stats) return launch_trace_wide<false, true, false>(bvh, r4, n, h4, st, pool, none, stream);
+        // (one launch over a small tree, as a tiny one's once its rays are not spread: 150,000 over 1,002
+        // leaves 53 us with a tail, 49 without)
+        const bool tail = share.tail && (n <= share.spread || bvh->wide_capacity > kWideSmallTree);
+        return tail ? launch_trace_wide<false, false, true>(bvh, r4, n, h4, st, pool, share, stream)
+                    : launch_trace_wide<false, false, false>(bvh, r4, n, h4, st, pool, none, stream);
     }
     if (any_hit) return stats ? launch_trace<true, true>(nd, r4, n, h4, st, pool, bvh->status, mv, stream)
                               : launch_trace<true, false>(nd, r4, n, h4, st, pool, bvh->status, mv, stream);

@@ -696,13 +696,42 @@ __device__ __forceinline__ bool wide_test_now(const WideState& s, bool live)
 // Lanes of a warp that take rays from the pool of n: all, or, where the grid has more
 // lanes than there are rays, the grid's even share, so that every warp has rays and the
 // lanes left over help with them (wide_tail); at least kWideMinLanes of them, because a
-// warp's step costs the same for one ray as for eight (1.3 M-triangle hairball scene, a
+// warp's step costs the same for one ray as for eight (in an early form, 1.3 M-triangle hairball scene, a
 // launch of 1,000 / 10,000 / 60,000 rays: 256 / 350 / 488 us with 1, 223 / 315 / 486 with
 // 4, 186 / 291 / 489 with 8, 237 / 324 / 492 with 16, 263 / 375 / 504 with all 32; without
 // helpers 387 / 739 / 1,231 us). Launches size their grids by it.
 constexpr uint32_t kWideMinLanes = 8;
-__device__ __forceinline__ uint32_t wide_ray_lanes(uint32_t n)
+// What a launch shares, by the leaves of its (largest) tree: with `tail` its last rays, and it
+// spreads its rays as above if they are `spread` at most. Helpers pay where the slowest rays are
+// much longer than the average one, and eight rays a warp where the chip has issue slots to
+// spare for it: in a large tree always, in a smaller one until the rays fill an eighth of the
+// chip's lanes, in a tiny one never. Closest hits of 1,000 / 34,440 / 80,000 rays, in us:
+//   leaves      nothing shared       spread           not spread
+//       202    16.9 / 20.0 /  24   18.9 / 29.2 /  33   19.4 / 21.5 /  27
+//     1,002    28.2 / 31.6 /  41   23.6 / 38.8 /  44   28.7 / 31.4 /  38
+//     3,026    51.7 / 59.8 /  73   41.5 / 75.7 /  89   51.2 / 54.7 /  76  (hairballs from here)
+//    11,026    90.6 / 99.3 / 124   59.9 /  112 / 133   67.1 / 86.5 / 121
+//    51,026     212 /  248 / 320    103 /  214 / 293    146 /  202 / 288
+//   201,026     592 /  685 / 904    239 /  498 / 743    386 /  552 / 769
+// Frames (512 leaves up, any size) gain by sharing throughout.
+struct WideShare {
+    bool tail;
+    uint32_t spread;
+};
+constexpr uint32_t kWideTinyTree = 512, kWideSmallTree = 2048, kWideLargeTree = 65536;
+inline WideShare wide_share(uint32_t leaves, int sms)
 {
+    if (leaves <= kWideTinyTree) return {false, 0u};
+    return {true, leaves <= kWideLargeTree ? (uint32_t)sms * 1024u / kWideMinLanes : 0xFFFFFFFFu};
+}
+// Rays that a block of such a launch takes at first.
+inline uint32_t wide_block_rays(WideShare share, uint32_t n, uint32_t block)
+{
+    return n <= share.spread ? kWideMinLanes * (block / 32u) : block;
+}
+__device__ __forceinline__ uint32_t wide_ray_lanes(uint32_t n, uint32_t spread)
+{
+    if (n > spread) return 32u;
     const uint32_t warps = gridDim.x * (blockDim.x / 32u);
     return min(32u, max(kWideMinLanes, n / warps + (n % warps != 0u)));
 }
@@ -969,13 +998,13 @@ struct WideHits {
 // direction's .w. Same refill rule and far-limit convention as persistent_trace.
 // sink.hit(ray, t, u, v, triangle) is called for every nearer hit, sink.done(ray, state) once
 // at the ray's end; sink.found(ray) is the triangle of the last hit given to sink.hit. kTail:
-// the launch's end shares rays among lanes (wide_tail).
+// the launch's end shares rays among lanes (wide_tail); spread: see wide_ray_lanes.
 template <bool kAny, int kBlock, bool kStats, int kSteps, bool kTmax, bool kTail, typename WideOf, typename Sink>
 __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const float4* __restrict__ rays, uint32_t n,
                                                       uint32_t* __restrict__ pool, uint2* smem_col, bool& overflow,
                                                       uint32_t& n_nodes, uint32_t& n_tris,
                                                       const uint32_t* __restrict__ order, Sink sink,
-                                                      uint32_t refill = 0)
+                                                      uint32_t spread, uint32_t refill = 0)
 {
     const uint32_t refill_below = refill ? refill : (uint32_t)kWideRefillLanes;
     const uint32_t lane = threadIdx.x & 31u;
@@ -987,7 +1016,7 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
     uint32_t ray = CPT_INVALID_INDEX;
     bool drained = false;
     static_assert(!kTail || kAny || !kTmax, "a ray traced anew starts unbounded");
-    const uint32_t lanes = kTail ? wide_ray_lanes(n) : 32u;
+    const uint32_t lanes = kTail ? wide_ray_lanes(n, spread) : 32u;
     // one grab per warp takes all the rays
     const bool once = kTail && n <= lanes * (gridDim.x * (blockDim.x / 32u));
     for (;;) {
