@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kMortonBlock) k_morton(const float* __restrict
 // subtrees inside each block of leaves, then the nodes across blocks.
 // ---------------------------------------------------------------------------
 template <typename K>
-__global__ void __launch_bounds__(kTreeBlock, 5) k_tree_blocks(TreeArrays<K> T, TriangleLeaves leaf, TreeList list)
+__global__ void __launch_bounds__(kTreeBlock, kTreeBlocks) k_tree_blocks(TreeArrays<K> T, TriangleLeaves leaf, TreeList list)
 {
     __shared__ TreeSmem sm;
     wait_for_previous();

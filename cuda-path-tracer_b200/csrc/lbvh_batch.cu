@@ -157,7 +157,7 @@ __device__ __forceinline__ TriangleLeaves batch_leaves(const BatchTable& bt, uin
 }
 
 template <typename K>
-__global__ void __launch_bounds__(kTreeBlock, 5) k_batch_tree_blocks(BatchTable bt, const uint32_t* __restrict__ order,
+__global__ void __launch_bounds__(kTreeBlock, kTreeBlocks) k_batch_tree_blocks(BatchTable bt, const uint32_t* __restrict__ order,
                                                                   int* __restrict__ ends, TreeList list,
                                                                   const uint32_t* __restrict__ batch_status)
 {
@@ -309,6 +309,8 @@ int batch_impl(BatchTable& bt, const cpt_triangle* const* tris_in, cpt_bvh* cons
     const uint32_t blocks = bt.block_off[bt.scenes];
     {
         CPT_PROF(K_TOPOLOGY, stream);
+        CPT_CUDA_TRY(cudaFuncSetAttribute(k_batch_tree_blocks<K>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          kTreeCarveout));
         launch_early(start_early(bt.total), k_batch_tree_blocks<K>, blocks, kTreeBlock, 0, stream, bt, order,
                      s.counters, list, s.status);
     }

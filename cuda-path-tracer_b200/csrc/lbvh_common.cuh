@@ -121,19 +121,23 @@ __device__ __forceinline__ int arrive_acq_rel(int* counter)
 //
 // 5.24 M triangles (1.22 GB of DRAM traffic): 724 us as a launch of key searches per node and
 // a walk per leaf through the records in memory (a third of the lanes left at every level, 25 %
-// of issue slots used); now 442 + 114. What bounds tree_block is shared memory (57 % of its
-// wavefronts) and five blocks' barriers; blocks of 128 leaves take 40 us less there and 43 more
-// above. tree_climb is a chain of about 20 steps of 2 us, a release, an exchange and the
-// sibling's box each, so small trees gain least (65,538 triangles: 61 us against 58).
+// of issue slots used); now 482 + 122. What bounds tree_block is shared memory (65 % of the L1
+// pipe's time) and the barriers and loads that three blocks an SM cannot hide (five: 428); blocks
+// of 128 leaves took 40 us less there and 43 more above. tree_climb is a chain of about 20 steps
+// of 2 us, a release, an exchange and the sibling's box each, so small trees gain least (65,538
+// triangles: 61 us as the former launches, 58 as these).
 // ---------------------------------------------------------------------------
 constexpr int kTreeBlock = 256;
 constexpr int kTreeLevels = 9;  // tables of 1, 2, ... 256 in a row
 constexpr int kNoEnd = -1;      // ends[g]: no child of split g has arrived
-// Percent of an SM's shared memory that the tree kernels ask for: four blocks instead of five, so
-// that the split is the renderer's and an SM that traces on another stream need not fall idle to
-// change it (C2 frames with the next scene's builds beside them: 135.9 ms a step with five blocks,
-// 122.2 with 71 %, 122.5 with 57 %; the build alone 1.30, 1.35 and 1.35 ms in the same program).
-constexpr int kTreeCarveout = 71;
+// The tree kernels run three blocks an SM, in the 132 KB split of the shared memory that the
+// renderer's traversal has too: an SM that traces on another stream then need not fall idle to
+// change it. Frames of C2 with the next scene's builds beside them take 122.8 ms a step with
+// three blocks, 136 to 139 with four (196 KB) and 136 with five (228 KB); 5.24 M triangles alone
+// 1,275, 1,223 and 1,213 us.
+constexpr int kTreeBlocks = 3;
+constexpr int kTreeSplitKb = 132;
+constexpr int kTreeCarveout = 100 * kTreeSplitKb / 228;  // percent of the most (228 KB), as the driver is asked for it
 constexpr int kTreeListWord = 16;  // the list's count among the 32 zeroed tile counters (a sort uses 9 at most)
 
 // Blocks of 128 threads for tree_climb over the subtrees of `blocks` blocks (a grid-stride
@@ -188,6 +192,9 @@ __device__ __forceinline__ float4 record_meta(uint32_t g, bool left_internal, bo
     const uint32_t word = (g << 2) | (right_internal ? 2u : 0u) | (left_internal ? 1u : 0u);
     return make_float4(__uint_as_float(word), __uint_as_float(g + 1u), __uint_as_float(far_end), 0.0f);
 }
+
+// (1 KB of each block is the system's)
+static_assert(kTreeBlocks * (sizeof(TreeSmem) + 1024) <= kTreeSplitKb * 1024, "the blocks fit the split");
 
 // The leaves [base, base + count) of tree T (count <= kTreeBlock threads' worth; all of the
 // block's threads call). leaf.load(i, slot, box) gives leaf i's child slot and box and writes

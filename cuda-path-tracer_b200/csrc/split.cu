@@ -466,7 +466,7 @@ struct PieceLeaves {
 // The split tree over *n_pieces sorted pieces (lbvh_common.cuh); node_cap: the records of
 // `nodes`, those past the tree marked unused.
 template <typename K>
-__global__ void __launch_bounds__(kTreeBlock, 5) k_split_tree_blocks(TreeArrays<K> T, PieceLeaves leaf, TreeList list,
+__global__ void __launch_bounds__(kTreeBlock, kTreeBlocks) k_split_tree_blocks(TreeArrays<K> T, PieceLeaves leaf, TreeList list,
                                                                   const uint32_t* __restrict__ n_pieces,
                                                                   uint32_t node_cap)
 {
