@@ -309,9 +309,14 @@ __global__ void __launch_bounds__(kExtendBlock, CPT_EXTEND_MIN_BLOCKS) k_extend(
             tr = vs.v[vi].wide_tris;
             return vs.v[vi].wide_nodes;
         };
-        persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false, kTail>(
-            wide_of, queue, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, order,
-            WideHits{hits}, spread, refill ? refill : kOneView ? (uint32_t)kWideRefillLanes : (uint32_t)kViewsRefillLanes);
+        const uint32_t refill_below = refill ? refill : kOneView ? (uint32_t)kWideRefillLanes : (uint32_t)kViewsRefillLanes;
+        auto run = [&](auto sink) {
+            persistent_trace_wide<false, kExtendBlock, kStats, kExtendSteps, false, kTail>(
+                wide_of, queue, n, pool, reinterpret_cast<uint2*>(s_stack) + threadIdx.x, overflow, nn, nt, order, sink,
+                spread, refill_below);
+        };
+        if constexpr (kTail) run(WideHits{hits});
+        else run(WideHitsAtEnd(hits));
         if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
         if (kStats && ray_counts) {
             warp_count_u64(ray_counts + 3, nn);

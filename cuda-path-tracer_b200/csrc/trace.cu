@@ -30,25 +30,14 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace(const float4* __restrict_
     if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
 }
 
-// Hits, and with kStats each ray's (node fetches, triangle tests). A visibility ray ends with
-// its first hit, so hits and misses are written together, at the end (in turn, 1 to 3 M of them
-// over 11,026 to 641,026 triangles took 2 to 9 % longer).
-template <bool kAny, bool kStats> struct TraceSink : WideHits {
+// Hits, and each ray's (node fetches, triangle tests).
+struct TraceStats : WideHitsAtEnd {
     uint2* stats;
-    mutable float4 first;
-    __device__ __forceinline__ TraceSink(float4* h, uint2* s) : WideHits{h}, stats(s) {}
-    __device__ __forceinline__ void hit(uint32_t ray, float t, float u, float v, float tri) const
-    {
-        if (kAny) first = make_float4(t, u, v, tri);
-        else WideHits::hit(ray, t, u, v, tri);
-    }
+    __device__ __forceinline__ TraceStats(float4* h, uint2* s) : WideHitsAtEnd(h), stats(s) {}
     __device__ __forceinline__ void done(uint32_t ray, const WideState& s) const
     {
-        if (kAny)
-            hits[ray] = s.t == kWideFound ? first : make_float4(FLT_MAX, 0.f, 0.f, __uint_as_float(CPT_INVALID_INDEX));
-        else
-            WideHits::done(ray, s);
-        if (kStats && stats) stats[ray] = make_uint2(s.visits, s.tests);
+        WideHitsAtEnd::done(ray, s);
+        if (stats) stats[ray] = make_uint2(s.visits, s.tests);
     }
 };
 
@@ -56,10 +45,10 @@ template <bool kAny, bool kStats> struct TraceSink : WideHits {
 // compiler takes 74 to 85 registers, 5 or 6 blocks, and the latency of the node fetches shows
 // (one million incoherent rays: 3.8 ms at 6 blocks, 2.5 at 8). Where nothing is shared
 // (visibility, counts, tiny trees) a launch of 150,000 to 300,000 rays lasts 5 to 20 % longer
-// when all fit at once than when lanes refill: 7 blocks, 6 for tiny trees (150,000 visibility rays over 1.2 M triangles 5.46 ms
+// when all fit at once than when lanes refill: 7 blocks for visibility, else 6 (150,000 visibility rays over 1.2 M triangles 5.46 ms
 // at 8, 5.01 at 7, 4.79 at 6; 1,000,003 of them 14.0, 13.9 and 14.3).
 template <bool kAny, bool kStats, bool kTail>
-__global__ void __launch_bounds__(kTraceBlock, kTail ? 8 : kAny || kStats ? 7 : 6) k_trace_wide(const float4* __restrict__ nodes,
+__global__ void __launch_bounds__(kTraceBlock, kTail ? 8 : kAny ? 7 : 6) k_trace_wide(const float4* __restrict__ nodes,
                                                             const float4* __restrict__ tris, uint32_t node_cap,
                                                             const float4* __restrict__ rays, uint32_t n,
                                                             float4* __restrict__ hits, uint2* __restrict__ stats,
@@ -74,9 +63,13 @@ __global__ void __launch_bounds__(kTraceBlock, kTail ? 8 : kAny || kStats ? 7 : 
         tr = tris;
         return nodes;
     };
-    persistent_trace_wide<kAny, kTraceBlock, kStats, kTraceSteps, false, kTail>(
-        wide_of, rays, n, pool, s_stack + threadIdx.x, overflow, nn, nt, nullptr,
-        TraceSink<kAny, kStats>(hits, stats), spread);
+    auto run = [&](auto sink) {
+        persistent_trace_wide<kAny, kTraceBlock, kStats, kTraceSteps, false, kTail>(
+            wide_of, rays, n, pool, s_stack + threadIdx.x, overflow, nn, nt, nullptr, sink, spread);
+    };
+    if constexpr (kStats) run(TraceStats(hits, stats));
+    else if constexpr (kTail) run(WideHits{hits});
+    else run(WideHitsAtEnd(hits));
     if (overflow) atomicOr(status, CPT_STATUS_STACK_OVERFLOW);
 }
 

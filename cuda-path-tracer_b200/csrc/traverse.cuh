@@ -993,6 +993,24 @@ struct WideHits {
     __device__ __forceinline__ uint32_t found(uint32_t ray) const { return __float_as_uint(hits[ray].w); }
 };
 
+// The same, each ray's written at its end: a lane that shares nothing keeps its hit until then, so
+// that a warp's hits and misses are stored together (visibility rays, whose first hit is the last:
+// 1 to 3 M over 11,026 to 641,026 triangles took 2 to 9 % longer when written as found; frames
+// over 302 triangles 1 to 4 %).
+struct WideHitsAtEnd {
+    float4* hits;
+    mutable float4 best;
+    __device__ __forceinline__ WideHitsAtEnd(float4* h) : hits(h) {}
+    __device__ __forceinline__ void hit(uint32_t, float t, float u, float v, float tri) const
+    {
+        best = make_float4(t, u, v, tri);
+    }
+    __device__ __forceinline__ void done(uint32_t ray, const WideState& s) const
+    {
+        hits[ray] = s.t == FLT_MAX ? make_float4(FLT_MAX, 0.f, 0.f, __uint_as_float(CPT_INVALID_INDEX)) : best;
+    }
+};
+
 // persistent_trace over wide BVHs: wide_of(w, max_visits, tris) returns the wide
 // node array, its node capacity and its triangle records for the word w of the
 // direction's .w. Same refill rule and far-limit convention as persistent_trace.
@@ -1065,9 +1083,11 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
             if ((kTail || !drained) && ((uint32_t)__popc(live) < refill_below || k >= kSteps)) break;
         }
     }
-    if (kTail && __ballot_sync(0xFFFFFFFFu, ray != CPT_INVALID_INDEX) != 0u) {
-        __shared__ WideTail s_tail[kBlock / 32];
-        overflow |= wide_tail<kAny, kBlock>(s, ray, smem_col, spill, s_perm, s_tail[threadIdx.x >> 5], sink);
+    if constexpr (kTail) {
+        if (__ballot_sync(0xFFFFFFFFu, ray != CPT_INVALID_INDEX) != 0u) {
+            __shared__ WideTail s_tail[kBlock / 32];
+            overflow |= wide_tail<kAny, kBlock>(s, ray, smem_col, spill, s_perm, s_tail[threadIdx.x >> 5], sink);
+        }
     }
 }
 
