@@ -271,8 +271,8 @@ __global__ void __launch_bounds__(kGenBlock) k_generate(Wave wv, Views vs, float
 }
 
 // A refill of rays of several views loads each ray's tree as well, so it waits for more lanes
-// than one of a single scene (kWideRefillLanes; twelve scenes of 5,000 to 50,000 triangles:
-// 10.2 ms a frame at 31, 9.9 at 28, 10.1 at 24).
+// than one of a single scene (kWideRefillLanes; twelve scenes of 10,000 to 500,000 triangles
+// built and rendered: 10.2 ms at 31, 9.9 at 28, 10.1 at 24).
 constexpr int kViewsRefillLanes = 28;
 
 // kOneView: every ray traverses view 0's BVH (a single scene, e.g. several cameras of

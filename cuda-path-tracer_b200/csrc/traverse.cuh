@@ -696,11 +696,12 @@ __device__ __forceinline__ bool wide_test_now(const WideState& s, bool live)
 // Lanes of a warp that take rays from the pool of n: all, or, where the grid has more
 // lanes than there are rays, the grid's even share, so that every warp has rays and the
 // lanes left over help with them (wide_tail); at least kWideMinLanes of them, because a
-// warp's step costs the same for one ray as for eight (in an early form, 1.3 M-triangle hairball scene, a
-// launch of 1,000 / 10,000 / 60,000 rays: 256 / 350 / 488 us with 1, 223 / 315 / 486 with
-// 4, 186 / 291 / 489 with 8, 237 / 324 / 492 with 16, 263 / 375 / 504 with all 32; without
+// warp's step costs the same for one ray as for eight (in an early form, over a 1.3 M-triangle
+// hairball scene, a launch of 1,000 / 10,000 / 60,000 rays: 256 / 350 / 488 us with 1, 223 / 315 /
+// 486 with 4, 186 / 291 / 489 with 8, 237 / 324 / 492 with 16, 263 / 375 / 504 with all 32; without
 // helpers 387 / 739 / 1,231 us). Launches size their grids by it.
 constexpr uint32_t kWideMinLanes = 8;
+
 // What a launch shares, by the leaves of its (largest) tree: with `tail` its last rays, and it
 // spreads its rays as above if they are `spread` at most. Helpers pay where the slowest rays are
 // much longer than the average one, and eight rays a warp where the chip has issue slots to
@@ -724,11 +725,13 @@ inline WideShare wide_share(uint32_t leaves, int sms)
     if (leaves <= kWideTinyTree) return {false, 0u};
     return {true, leaves <= kWideLargeTree ? (uint32_t)sms * 1024u / kWideMinLanes : 0xFFFFFFFFu};
 }
+
 // Rays that a block of such a launch takes at first.
 inline uint32_t wide_block_rays(WideShare share, uint32_t n, uint32_t block)
 {
     return n <= share.spread ? kWideMinLanes * (block / 32u) : block;
 }
+
 __device__ __forceinline__ uint32_t wide_ray_lanes(uint32_t n, uint32_t spread)
 {
     if (n > spread) return 32u;
@@ -746,14 +749,15 @@ __device__ __forceinline__ uint32_t wide_ray_lanes(uint32_t n, uint32_t spread)
 // nearest distance (t, indexed by the ray's lane), so each prunes with what any of them has
 // found. A ray is finished when its own lane and all its helpers are.
 //
-// Measured (before -> after): C1's frame 1,008 -> 808 us, a 1280x720 one-sample frame with
-// shadow rays 6.1 -> 3.6 ms, one million incoherent rays 3.7 -> 3.0 ms, 10,000 of them 740 ->
-// 250 us, C2's 16-sample frame 94.9 -> 93.3 ms. Thresholds 8 / 12 / 16 lanes: 809 / 789 / 786
+// Measured (without -> with): C1's frame 1,003 -> 795 us, a 1280x720 one-sample frame with
+// shadow rays 6.0 -> 3.4 ms, one million incoherent rays 3.6 -> 2.9 ms, 12,000 rays over 201,026
+// triangles 645 -> 327 us, C2's 16-sample frame 95.2 -> 94.0 ms. Thresholds 8 / 12 / 16 lanes: 809 / 789 / 786
 // us and 4.52 / 4.37 / 4.37 ms on the first two in an earlier form; 28 and 31 lose (helpers
 // visit nodes that a nearer hit would have culled). It is a function of its own, called with
 // a copy of the state, because the loop before it has no register to spare: inlined, or with
 // the state live across the loop's end, C2 ran 5 to 8 % slower. For the same reason a hit is
-// written when it is found instead of carried (u, v, triangle) to the ray's end.
+// written when it is found instead of carried (u, v, triangle) to the ray's end. (It spills 112
+// to 118 B itself, 64 to 68 B for shadow rays.)
 //
 // The hit is the one that a lane finds alone, one visit after the other. Which boxes are passed
 // over depends on what has been found by then, and the distance that tri_test computes for a
@@ -783,7 +787,7 @@ struct WideTail {  // per warp, in shared memory; t to other by the ray's lane
     float other[32];    // the nearest distance of another triangle
     uint32_t info[32];  // byte 0: helpers at work; byte 1 (of word r): the r-th lane with a stack entry to give
 };
-constexpr float kWideBehind = 1.0f + 1.0f / 64.0f;  // (1/256 costs as much; 0: 3 of 640,000 rays differ from 400 units)
+constexpr float kWideBehind = 1.0f + 1.0f / 64.0f;  // (1/256 costs as much; 0: 4 of 640,000 rays from 400 units differ)
 constexpr int kWideSpill = CPT_TRAVERSAL_STACK - kWideSmemStack;
 // A lane's words that are rarely touched: in local memory, behind its stack, so that they hold no
 // register while a node is visited.
@@ -1086,11 +1090,13 @@ __device__ __forceinline__ void persistent_trace_wide(WideOf wide_of, const floa
     if constexpr (kTail) {
         if (__ballot_sync(0xFFFFFFFFu, ray != CPT_INVALID_INDEX) != 0u) {
             __shared__ WideTail s_tail[kBlock / 32];
+            static_assert((1024 / kBlock) * (kWideSmemStack * kBlock * sizeof(uint2) + sizeof(s_perm) + sizeof(s_tail) + 1024) <=
+                              132 * 1024,
+                          "1,024 threads an SM stay within the 132 KB split (1 KB of each block is the system's)");
             overflow |= wide_tail<kAny, kBlock>(s, ray, smem_col, spill, s_perm, s_tail[threadIdx.x >> 5], sink);
         }
     }
 }
-
 
 // persistent_trace of unbounded rays whose hit goes to hits[i] = (t, u, v, triangle).
 // ray_stats (nullable, with kStats): per ray (node fetches, triangle tests).
