@@ -317,7 +317,11 @@ int cpt_render_views(const cpt_view* views, uint32_t n_views, const cpt_render_p
  * copies the leaf triangles into 48-B records in visiting order (two record positions
  * per binary leaf are reserved). Tracing and rendering then traverse it.
  * Hits are those of the binary tree (same triangle arithmetic) up to which of several
- * exactly equal distances is reported. `leaves` for the sizes: bvh->n, or
+ * exactly equal distances is reported, and up to rounding: the distance computed for a thin
+ * triangle seen from far away can lie before the box that holds it, and which of two such
+ * hits is found then depends on the tree (2 million rays over 400,000 hairs in a ball of
+ * radius 1.3: none differ from 3 units away, 4 from 20, 74 from 100, 889 from 400). A tree's
+ * hits do not depend on the launch. `leaves` for the sizes: bvh->n, or
  * bvh->split_capacity after cpt_lbvh_split. status[2] / status[3] receive the wide
  * node count and the record positions used. */
 #define CPT_WIDE_SAH 1u /* choose each wide node's children by a surface-area cost computed bottom-up over
