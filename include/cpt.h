@@ -320,8 +320,8 @@ int cpt_render_views(const cpt_view* views, uint32_t n_views, const cpt_render_p
  * exactly equal distances is reported, and up to rounding: the distance computed for a thin
  * triangle seen from far away can lie before the box that holds it, and which of two such
  * hits is found then depends on the tree (2 million rays over 400,000 hairs in a ball of
- * radius 1.3: none differ from 3 units away, 4 from 20, 74 from 100, 889 from 400). A tree's
- * hits do not depend on the launch. `leaves` for the sizes: bvh->n, or
+ * radius 1.3: none differ from 3 units away, 4 from 20, 74 from 100, 889 from 400). On
+ * the launch they depend for a few of ten million such rays at most. `leaves` for the sizes: bvh->n, or
  * bvh->split_capacity after cpt_lbvh_split. status[2] / status[3] receive the wide
  * node count and the record positions used. */
 #define CPT_WIDE_SAH 1u /* choose each wide node's children by a surface-area cost computed bottom-up over
